@@ -694,6 +694,22 @@ constexpr int kFluxHLL = 1, kFluxMC = 2;
 #define PGK_FLUX_MC(p) ((OPT & kFluxMC) != 0)
 #endif
 
+// The metric at a face. The FP64 kernels load it before they reconstruct, so
+// that its loads' latency passes meanwhile; the mixed form loads it in face_flux.
+struct FaceGeo {
+#if !PGK_MIXED
+  Geo g;
+  int ok;
+#endif
+};
+template <int MT, int DIR>
+__device__ __forceinline__ void face_geo(const Dims &d, const pangu_params &p, int b, int k, int j,
+                                         int i, FaceGeo &fg) {
+#if !PGK_MIXED
+  fg.ok = face_metric<MT>(d, p, DIR, b, k, j, i, fg.g);
+#endif
+}
+
 // Reconstruction of one variable in cell q (stride s along the direction):
 // ql_ip1 = value at the upper face, qr_i = value at the lower face
 // (interpolater_mc.h:38-48, interpolater_ppm4.h:29-67).
@@ -714,26 +730,173 @@ __device__ __forceinline__ void recon_cell(bool use_mc, const PT *q, long long s
 #endif
 }
 
-// One flux component from a state (contravariant_flux.h:12-39).
-template <int c>
-__device__ __forceinline__ double flux_component(double gam, const double P[NPRIM],
-                                                 const State &s, double sg, int dir) {
-  const double f_rho = P[RHO] * s.ucon[dir];
-  if (c == RHO) return f_rho * sg;
-  if (c == ENT) return (P[ENT] * f_rho) * sg;
-  if (c == KEL) return (P[KEL] * f_rho) * sg;
-  if (c >= BX1 && c <= BX3) {
-    const int m = c - BX1 + 1;
-    return SUB(MUL(s.bcon[m], s.ucon[dir]), MUL(s.bcon[dir], s.ucon[m])) * sg;
+// Reconstruction of every variable in one cell: cell(v) points at component v
+// of the cell (stride s along the direction) and put(s, up, lo) takes variable
+// s's upper- and lower-face values.
+template <int OPT, class Cell, class Put>
+__device__ __forceinline__ void recon_vars(const Dims &d, const pangu_params &p, Cell cell,
+                                           long long st, Put put) {
+#if !PGK_MIXED
+  if (!(OPT & kFluxMC)) {
+    unsigned redo = 0;  // variables outside ppm4_face's range
+#pragma unroll
+    for (int s = 0; s < NPRIM; ++s) {
+      FT up = 0, lo = 0;
+      bool ok = true;
+      if (d.pidx[s] >= 0) {
+        const PT *q = cell(d.pidx[s]);
+        const double m1 = q[-st], q0 = q[0], p1 = q[st];
+        const double fl = ppm4_face(q[-2 * st], m1, q0, p1, ok);
+        const double fu = ppm4_face(m1, q0, p1, q[2 * st], ok);
+        up = ppm4_side(q0, fl, fu);
+        lo = ppm4_side(q0, fu, fl);
+      }
+      put(s, up, lo);
+      if (!ok) redo |= 1u << s;
+    }
+    if (redo) {
+#pragma unroll
+      for (int s = 0; s < NPRIM; ++s)
+        if (redo >> s & 1u) {
+          const double2 r = ppm4_plain(cell(d.pidx[s]), st);
+          put(s, r.x, r.y);
+        }
+    }
+    return;
   }
-  const double hh = P[RHO] + gam * P[ENY];
-  const double e_tot = hh + s.bsq;
-  const double p_tot = (gam - 1.) * P[ENY] + 0.5 * s.bsq;
-  const int m = (c == ENY) ? 0 : c - UX1 + 1;
-  const double t = e_tot * s.ucon[dir] * s.ucov[m] + p_tot * (dir == m) - s.bcon[dir] * s.bcov[m];
-  if (c == ENY) return (t + f_rho) * sg;
-  return t * sg;
+#endif
+#pragma unroll
+  for (int s = 0; s < NPRIM; ++s) {
+    FT up = 0, lo = 0;
+    if (d.pidx[s] >= 0) recon_cell(PGK_FLUX_MC(p), cell(d.pidx[s]), st, up, lo);
+    put(s, up, lo);
+  }
 }
+
+// Reconstruction of every variable along x1 by a warp whose lane l holds cell
+// c0 + l: as recon_vars, but each face value of PPM4 is formed once and handed
+// to the next lane. The lower face of lane 0's cell is formed for component l
+// by lane l, through `edge` (shared memory, NPRIM entries of this warp).
+// cell(v, l) points at component v of lane l's cell; the stencils of inactive
+// lanes have to be readable.
+template <int OPT, class Cell, class Put>
+__device__ __forceinline__ void recon_row(const Dims &d, const pangu_params &p, Cell cell, int lane,
+                                          bool active, FT *edge, Put put) {
+#if !PGK_MIXED
+  if (!(OPT & kFluxMC)) {
+    if (lane < d.NF) {
+      const PT *q = cell(lane, 0);
+      bool ok = true;
+      double v = ppm4_face(q[-2], q[-1], q[0], q[1], ok);
+      if (!ok) v = ppm4_face_plain(q[-2], q[-1], q[0], q[1]);
+      edge[lane] = v;
+    }
+    __syncwarp();
+    unsigned redo = 0;  // variables whose upper-face value is outside ppm4_face's range
+#pragma unroll
+    for (int s = 0; s < NPRIM; ++s) {
+      FT up = 0, lo = 0;
+      bool ok = true;
+      if (d.pidx[s] >= 0) {
+        const PT *q = cell(d.pidx[s], lane);
+        const double q0 = q[0];
+        const double fu = ppm4_face(q[-1], q0, q[1], q[2], ok);
+        double fl = __shfl_up_sync(0xffffffffu, fu, 1);
+        if (lane == 0) fl = edge[d.pidx[s]];
+        up = ppm4_side(q0, fl, fu);
+        lo = ppm4_side(q0, fu, fl);
+      }
+      put(s, up, lo);
+      if (!ok) redo |= 1u << s;
+    }
+    const unsigned prev = __shfl_up_sync(0xffffffffu, redo, 1);
+    if (lane > 0) redo |= prev;
+    if (redo && active) {
+#pragma unroll
+      for (int s = 0; s < NPRIM; ++s)
+        if (redo >> s & 1u) {
+          const double2 r = ppm4_plain(cell(d.pidx[s], lane), 1);
+          put(s, r.x, r.y);
+        }
+    }
+    return;
+  }
+#endif
+#pragma unroll
+  for (int s = 0; s < NPRIM; ++s) {
+    FT up = 0, lo = 0;
+    if (d.pidx[s] >= 0 && active) recon_cell(PGK_FLUX_MC(p), cell(d.pidx[s], lane), 1, up, lo);
+    put(s, up, lo);
+  }
+}
+
+#if !PGK_MIXED
+// Fluxes along DIR (or the conserved variables, DIR 0) of one state
+// (contravariant_flux.h:12-39): the products that every component shares, then
+// component c. Components whose row of p_tot delta is off the diagonal add
+// p_tot * 0 (zp), which keeps the reference's result where p_tot is not finite.
+template <int DIR>
+struct FluxOf {
+  double f_rho, eu, p_tot, zp;
+  __device__ __forceinline__ FluxOf(double gam, const double P[NPRIM], const State &s) {
+    f_rho = P[RHO] * s.ucon[DIR];
+    const double e_tot = P[RHO] + gam * P[ENY] + s.bsq;
+    p_tot = (gam - 1.) * P[ENY] + 0.5 * s.bsq;
+    zp = p_tot * 0.0;
+    eu = e_tot * s.ucon[DIR];
+  }
+  template <int c>
+  __device__ __forceinline__ double get(const double P[NPRIM], const State &s, double sg) const {
+    if (c == RHO) return f_rho * sg;
+    if (c == ENT) return (P[ENT] * f_rho) * sg;
+    if (c == KEL) return (P[KEL] * f_rho) * sg;
+    if (c >= BX1 && c <= BX3) {
+      const int m = c - BX1 + 1;
+      return SUB(MUL(s.bcon[m], s.ucon[DIR]), MUL(s.bcon[DIR], s.ucon[m])) * sg;
+    }
+    const int m = (c == ENY) ? 0 : c - UX1 + 1;
+    const double t = eu * s.ucov[m] + (DIR == m ? p_tot : zp) - s.bcon[DIR] * s.bcov[m];
+    return (c == ENY ? t + f_rho : t) * sg;
+  }
+};
+
+// Calls f.template operator()<c>() for every component that the engine's fields
+// have, c its compile-time variable.
+template <class F>
+__device__ __forceinline__ void for_components(const Dims &d, F f) {
+  f(std::integral_constant<int, RHO>{});
+  f(std::integral_constant<int, ENY>{});
+  f(std::integral_constant<int, UX1>{});
+  f(std::integral_constant<int, UX2>{});
+  f(std::integral_constant<int, UX3>{});
+  if (d.pidx[BX1] >= 0) {
+    f(std::integral_constant<int, BX1>{});
+    f(std::integral_constant<int, BX2>{});
+    f(std::integral_constant<int, BX3>{});
+  }
+  f(std::integral_constant<int, ENT>{});
+  if (d.pidx[KEL] >= 0) f(std::integral_constant<int, KEL>{});
+}
+
+// State and signal speeds of one side of a face.
+template <int MT, int DIR>
+__device__ __forceinline__ void face_side(double gam, const double P[NPRIM], const Geo &g,
+                                          const xd::Rcp &al, bool al_ok, State &st, double &vmax,
+                                          double &vmin) {
+  const bool ok = state_speed<MT>(gam, P, g, al, DIR, st, vmax, vmin);
+  if (!(ok & al_ok)) {
+    const Geo gc = g;
+    double Pc[NPRIM], v[2];
+    State sc;
+#pragma unroll
+    for (int n = 0; n < NPRIM; ++n) Pc[n] = P[n];
+    side_plain<MT>(gam, Pc, &gc, DIR, &sc, v);
+    st = sc;
+    vmax = v[0];
+    vmin = v[1];
+  }
+}
+#endif
 
 #if PGK_MIXED
 // One flux component from a state in FT arithmetic (contravariant_flux.h:12-39).
@@ -760,9 +923,9 @@ __device__ __forceinline__ FT flux_component_t(FT gam, const FT P[NPRIM], const 
 // Riemann flux and fast speed at the lower face of (b, k, j, i) along DIR in
 // FT arithmetic; the metric is evaluated in FP64 and rounded once.
 template <int MT, int DIR, int OPT>
-__device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, int b, int k, int j,
-                                          int i, const FT PL[NPRIM], const FT PR[NPRIM],
-                                          double *F, double *alfven) {
+__device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, const FaceGeo &,
+                                          int b, int k, int j, int i, const FT PL[NPRIM],
+                                          const FT PR[NPRIM], double *F, double *alfven) {
   const long long fo = coff(d, k, j, i);
   GeoT<FT> g;
   int ok;
@@ -829,55 +992,90 @@ __device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, 
 #else
 // Riemann flux and fast speed at the lower face of (b, k, j, i) along DIR
 // from the left and right states.
-template <int MT, int DIR, int OPT>
-__device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, int b, int k, int j,
-                                          int i, const double PL[NPRIM], const double PR[NPRIM],
-                                          double *F, double *alfven) {
-  Geo g;
-  const long long fo = coff(d, k, j, i);
-  if (!face_metric<MT>(d, p, DIR, b, k, j, i, g)) {
-    // Singular code metric (theta = 0 exactly on a polar face): zero flux,
-    // zero speed (the reference reads an unwritten inverse here).
-    a_alfven(d, alfven, b, DIR - 1)[fo] = 0.0;
+//
+// Singular code metric (theta = 0 exactly on a polar face): zero flux, zero
+// speed (the reference reads an unwritten inverse there).
+__device__ __forceinline__ void face_singular(const Dims &d, int dir, int b, long long fo, double *F,
+                                              double *alfven) {
+  a_alfven(d, alfven, b, dir - 1)[fo] = 0.0;
 #pragma unroll
-    for (int s = 0; s < NPRIM; ++s)
-      if (d.pidx[s] >= 0) a_flux(d, F, b, d.pidx[s])[fo] = 0.0;
+  for (int s = 0; s < NPRIM; ++s)
+    if (d.pidx[s] >= 0) a_flux(d, F, b, d.pidx[s])[fo] = 0.0;
+}
+
+// The two sides' fluxes and conserved values combined, component by component:
+// left(c) and right(c) give {flux, conserved}. HLL's ten quotients share their
+// denominator.
+template <int OPT, class L, class R>
+__device__ __forceinline__ void face_combine(const Dims &d, int dir, int b, long long fo,
+                                             double vmaxL, double vminL, double vmaxR,
+                                             double vminR, L left, R right, double *F,
+                                             double *alfven) {
+  const double cmax = fabs(kmax(kmax(0., vmaxL), vmaxR));
+  const double cmin = fabs(kmax(kmax(0., -vminL), -vminR));
+  const double cms = kmax(cmax, cmin);
+  a_alfven(d, alfven, b, dir - 1)[fo] = cms;
+  if ((OPT & kFluxHLL) != 0) {
+    const double den = cmax + cmin + 1e-20;
+    unsigned redo = xd::in_range_den(den) ? 0u : ~0u;  // components to divide plainly
+    const xd::Rcp id = xd::rcp(den);
+    double n[NPRIM];
+    for_components(d, [&](auto C) {
+      constexpr int c = decltype(C)::value;
+      const double2 l = left(C), r = right(C);
+      n[c] = cmax * l.x + cmin * r.x - cmax * cmin * (r.y - l.y);
+      if (!xd::in_range0(n[c])) redo |= 1u << c;
+      a_flux(d, F, b, d.pidx[c])[fo] = xd::quot_s(n[c], id);
+    });
+    if (redo)
+      for_components(d, [&](auto C) {
+        constexpr int c = decltype(C)::value;
+        if (redo >> c & 1u) a_flux(d, F, b, d.pidx[c])[fo] = div_plain(n[c], den);
+      });
+  } else {
+    for_components(d, [&](auto C) {
+      constexpr int c = decltype(C)::value;
+      const double2 l = left(C), r = right(C);
+      a_flux(d, F, b, d.pidx[c])[fo] = 0.5 * (l.x + r.x - cms * (r.y - l.y));
+    });
+  }
+}
+
+template <int MT, int DIR, int OPT>
+__device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, const FaceGeo &fg,
+                                          int b, int k, int j, int i, const double PL[NPRIM],
+                                          const double PR[NPRIM], double *F, double *alfven) {
+  const Geo &g = fg.g;
+  const long long fo = coff(d, k, j, i);
+  if (!fg.ok) {
+    face_singular(d, DIR, b, fo, F, alfven);
     return;
   }
   const double gam = p.adiabatic_index;
   const double sg = g.sg;
-  State sL, sR;
-  calc_state<MT>(PL, g, sL);
-  calc_state<MT>(PR, g, sR);
-  double vmaxL, vminL, vmaxR, vminR;
-  fast_speed_from_state(gam, PL, g, sL, DIR, vmaxL, vminL);
-  fast_speed_from_state(gam, PR, g, sR, DIR, vmaxR, vminR);
-  const double cmax = fabs(kmax(kmax(0., vmaxL), vmaxR));
-  const double cmin = fabs(kmax(kmax(0., -vminL), -vminR));
-  const double cms = kmax(cmax, cmin);
-  a_alfven(d, alfven, b, DIR - 1)[fo] = cms;
-  const bool hll = PGK_FLUX_HLL(p);
-#define PGD_FACE_COMPONENT(C)                                                         \
-  if (d.pidx[C] >= 0) {                                                               \
-    const double fl = flux_component<C>(gam, PL, sL, sg, DIR);                        \
-    const double fr = flux_component<C>(gam, PR, sR, sg, DIR);                        \
-    const double ul = flux_component<C>(gam, PL, sL, sg, 0);                          \
-    const double ur = flux_component<C>(gam, PR, sR, sg, 0);                          \
-    a_flux(d, F, b, d.pidx[C])[fo] =                                                     \
-        hll ? (cmax * fl + cmin * fr - cmax * cmin * (ur - ul)) / (cmax + cmin + 1e-20) \
-            : 0.5 * (fl + fr - cms * (ur - ul));                                      \
+  xd::Rcp al{};
+  bool al_ok = true;
+  if (MT != MINKOWSKI) {
+    al = xd::rcp(g.alpha);
+    al_ok = xd::in_range_den(g.alpha);
   }
-  PGD_FACE_COMPONENT(RHO)
-  PGD_FACE_COMPONENT(ENY)
-  PGD_FACE_COMPONENT(UX1)
-  PGD_FACE_COMPONENT(UX2)
-  PGD_FACE_COMPONENT(UX3)
-  PGD_FACE_COMPONENT(BX1)
-  PGD_FACE_COMPONENT(BX2)
-  PGD_FACE_COMPONENT(BX3)
-  PGD_FACE_COMPONENT(ENT)
-  PGD_FACE_COMPONENT(KEL)
-#undef PGD_FACE_COMPONENT
+  State sL, sR;
+  double vmaxL, vminL, vmaxR, vminR;
+  face_side<MT, DIR>(gam, PL, g, al, al_ok, sL, vmaxL, vminL);
+  face_side<MT, DIR>(gam, PR, g, al, al_ok, sR, vmaxR, vminR);
+  const FluxOf<DIR> fL(gam, PL, sL), fR(gam, PR, sR);
+  const FluxOf<0> uL(gam, PL, sL), uR(gam, PR, sR);
+  face_combine<OPT>(
+      d, DIR, b, fo, vmaxL, vminL, vmaxR, vminR,
+      [&](auto C) {
+        constexpr int c = decltype(C)::value;
+        return make_double2(fL.template get<c>(PL, sL, sg), uL.template get<c>(PL, sL, sg));
+      },
+      [&](auto C) {
+        constexpr int c = decltype(C)::value;
+        return make_double2(fR.template get<c>(PR, sR, sg), uR.template get<c>(PR, sR, sg));
+      },
+      F, alfven);
 }
 
 // face_flux with the two sides evaluated one after the other through shared
@@ -887,44 +1085,34 @@ __device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, 
 // su, and the right side combines them with its own. Every value is the one
 // face_flux computes, from the same operations on the same operands.
 template <int MT, int DIR, int OPT>
-__device__ __forceinline__ void face_flux_split(const Dims &d, const pangu_params &p, int b, int k,
-                                                int j, int i, double *sl, const double *sr,
-                                                double *su, int ss, double *F, double *alfven) {
-  Geo g;
+__device__ __forceinline__ void face_flux_split(const Dims &d, const pangu_params &p,
+                                                const FaceGeo &fg, int b, int k, int j, int i,
+                                                double *sl, const double *sr, double *su, int ss,
+                                                double *F, double *alfven) {
+  const Geo &g = fg.g;
   const long long fo = coff(d, k, j, i);
-  if (!face_metric<MT>(d, p, DIR, b, k, j, i, g)) {
-    a_alfven(d, alfven, b, DIR - 1)[fo] = 0.0;
-#pragma unroll
-    for (int s = 0; s < NPRIM; ++s)
-      if (d.pidx[s] >= 0) a_flux(d, F, b, d.pidx[s])[fo] = 0.0;
+  if (!fg.ok) {
+    face_singular(d, DIR, b, fo, F, alfven);
     return;
   }
   const double gam = p.adiabatic_index;
   const double sg = g.sg;
+  const xd::Rcp al = xd::rcp(g.alpha);
+  const bool al_ok = xd::in_range_den(g.alpha);
   double vmaxL, vminL;
   {
     double P[NPRIM];
 #pragma unroll
     for (int s = 0; s < NPRIM; ++s) P[s] = sl[s * ss];
     State st;
-    calc_state<MT>(P, g, st);
-    fast_speed_from_state(gam, P, g, st, DIR, vmaxL, vminL);
-#define PGD_LEFT_COMPONENT(C)                                 \
-  if (d.pidx[C] >= 0) {                                       \
-    sl[C * ss] = flux_component<C>(gam, P, st, sg, DIR);      \
-    su[C * ss] = flux_component<C>(gam, P, st, sg, 0);        \
-  }
-    PGD_LEFT_COMPONENT(RHO)
-    PGD_LEFT_COMPONENT(ENY)
-    PGD_LEFT_COMPONENT(UX1)
-    PGD_LEFT_COMPONENT(UX2)
-    PGD_LEFT_COMPONENT(UX3)
-    PGD_LEFT_COMPONENT(BX1)
-    PGD_LEFT_COMPONENT(BX2)
-    PGD_LEFT_COMPONENT(BX3)
-    PGD_LEFT_COMPONENT(ENT)
-    PGD_LEFT_COMPONENT(KEL)
-#undef PGD_LEFT_COMPONENT
+    face_side<MT, DIR>(gam, P, g, al, al_ok, st, vmaxL, vminL);
+    const FluxOf<DIR> f(gam, P, st);
+    const FluxOf<0> u(gam, P, st);
+    for_components(d, [&](auto C) {
+      constexpr int c = decltype(C)::value;
+      sl[c * ss] = f.template get<c>(P, st, sg);
+      su[c * ss] = u.template get<c>(P, st, sg);
+    });
   }
   // the right side reads the left side's results back from shared memory
   asm volatile("" ::: "memory");
@@ -932,35 +1120,21 @@ __device__ __forceinline__ void face_flux_split(const Dims &d, const pangu_param
 #pragma unroll
   for (int s = 0; s < NPRIM; ++s) P[s] = sr[s * ss];
   State st;
-  calc_state<MT>(P, g, st);
   double vmaxR, vminR;
-  fast_speed_from_state(gam, P, g, st, DIR, vmaxR, vminR);
-  const double cmax = fabs(kmax(kmax(0., vmaxL), vmaxR));
-  const double cmin = fabs(kmax(kmax(0., -vminL), -vminR));
-  const double cms = kmax(cmax, cmin);
-  a_alfven(d, alfven, b, DIR - 1)[fo] = cms;
-  const bool hll = PGK_FLUX_HLL(p);
-#define PGD_RIGHT_COMPONENT(C)                                                        \
-  if (d.pidx[C] >= 0) {                                                               \
-    const double fl = sl[C * ss];                                                     \
-    const double fr = flux_component<C>(gam, P, st, sg, DIR);                         \
-    const double ul = su[C * ss];                                                     \
-    const double ur = flux_component<C>(gam, P, st, sg, 0);                           \
-    a_flux(d, F, b, d.pidx[C])[fo] =                                                     \
-        hll ? (cmax * fl + cmin * fr - cmax * cmin * (ur - ul)) / (cmax + cmin + 1e-20) \
-            : 0.5 * (fl + fr - cms * (ur - ul));                                      \
-  }
-  PGD_RIGHT_COMPONENT(RHO)
-  PGD_RIGHT_COMPONENT(ENY)
-  PGD_RIGHT_COMPONENT(UX1)
-  PGD_RIGHT_COMPONENT(UX2)
-  PGD_RIGHT_COMPONENT(UX3)
-  PGD_RIGHT_COMPONENT(BX1)
-  PGD_RIGHT_COMPONENT(BX2)
-  PGD_RIGHT_COMPONENT(BX3)
-  PGD_RIGHT_COMPONENT(ENT)
-  PGD_RIGHT_COMPONENT(KEL)
-#undef PGD_RIGHT_COMPONENT
+  face_side<MT, DIR>(gam, P, g, al, al_ok, st, vmaxR, vminR);
+  const FluxOf<DIR> f(gam, P, st);
+  const FluxOf<0> u(gam, P, st);
+  face_combine<OPT>(
+      d, DIR, b, fo, vmaxL, vminL, vmaxR, vminR,
+      [&](auto C) {
+        constexpr int c = decltype(C)::value;
+        return make_double2(sl[c * ss], su[c * ss]);
+      },
+      [&](auto C) {
+        constexpr int c = decltype(C)::value;
+        return make_double2(f.template get<c>(P, st, sg), u.template get<c>(P, st, sg));
+      },
+      F, alfven);
 }
 #endif
 
@@ -968,21 +1142,21 @@ __device__ __forceinline__ void face_flux_split(const Dims &d, const pangu_param
 // reconstructs cell c = f0 - 1 + l; face c takes its left state from lane
 // l - 1 (upper-face value of cell c - 1) and its right state from lane l.
 constexpr int kFacesPerWarp = 31;
-// Flux kernels holding both states of a face in registers: at most 128
-// registers (4 CTAs of 4 warps per SM, a few spills). For them, bounds of 3
-// CTAs (168 registers) and of 5 or 6 (96 or 80) were measured slower on the
-// 2D torus (the latter two faster on the 3D one).
+// Flux kernels run at 4 CTAs of 4 warps per SM (128 registers, few or no
+// spills). They are bound by issue and by FP64 latency: 28 % fewer instructions
+// per face than with a division per quotient and both face values per cell, so
+// what a fifth CTA (96 registers) would hide it now loses in spills (2D torus
+// 47 against 59 us for both directions, 3D torus 2.41 against 2.59 ms for
+// three; 3 CTAs with 168 registers: 56 us and 3.17 ms).
 constexpr int kFluxThreads = 128;
-// With one side's state in registers at a time (FP64, curved metrics) the
-// flux kernels run at 5 CTAs per SM (96 registers): measured 1.1 % faster per
-// cycle on the 2D and the 3D torus than both states at 4 CTAs (at 4 CTAs the
-// split alone gained nothing); on Minkowski (Orszag-Tang) it cost 1.6 %, so
-// it is not used there.
+constexpr int kFluxBlocks = 4;
+// FP64, curved metrics: one side's state in registers at a time
+// (face_flux_split; 47 against 49 us on the 2D torus, 2.41 against 2.52 ms on
+// the 3D one). Minkowski keeps both (its metric takes no registers).
 constexpr bool split_faces(int mt) { return PGK_SPLIT_FACES && mt != MINKOWSKI; }
-constexpr int flux_blocks(int mt) { return split_faces(mt) ? 5 : 4; }
 
 template <int MT, int OPT>
-__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT)) k_flux_x1(Dims d, pangu_params p, int k0, int k1,
+__global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_x1(Dims d, pangu_params p, int k0, int k1,
                                                       int j0, int j1, int i0, int i1,
                                                       const PT *P, double *F,
                                                       double *alfven) {
@@ -1002,7 +1176,11 @@ __global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT)) k_flux_x1(Dims 
   const int j = j0 + (int)jr;
   const int c = i0 - 1 + seg * kFacesPerWarp + lane;
   const bool active = c <= i1;  // cell c is needed by face c (and c + 1)
-  const bool use_mc = PGK_FLUX_MC(p);
+  __shared__ FT edge[kFluxThreads / 32][NPRIM];
+  // an inactive lane reads the last cell's stencil
+  auto cell = [&](int v, int l) {
+    return a_prim(d, P, b, v) + coff(d, k, j, min(c - lane + l, i1));
+  };
 #if PGK_SPLIT_FACES
   if (split_faces(MT)) {
     // [3][NPRIM][blockDim.x]: upper-face values, lower-face values, and the
@@ -1011,32 +1189,30 @@ __global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT)) k_flux_x1(Dims 
     // fluxes over them.
     extern __shared__ double fsm[];
     const int ss = blockDim.x, t = threadIdx.x;
-#pragma unroll
-    for (int s = 0; s < NPRIM; ++s) {
-      FT up = 0, lo = 0;
-      if (d.pidx[s] >= 0 && active)
-        recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, k, j, c), 1, up, lo);
+    recon_row<OPT>(d, p, cell, lane, active, edge[t >> 5], [&](int s, FT up, FT lo) {
       fsm[s * ss + t] = up;
       fsm[(NPRIM + s) * ss + t] = lo;
-    }
+    });
     __syncwarp();
     if (lane == 0 || !active) return;
-    face_flux_split<MT, 1, OPT>(d, p, b, k, j, c, fsm + t - 1, fsm + NPRIM * ss + t,
+    FaceGeo fg;
+    face_geo<MT, 1>(d, p, b, k, j, c, fg);
+    face_flux_split<MT, 1, OPT>(d, p, fg, b, k, j, c, fsm + t - 1, fsm + NPRIM * ss + t,
                            fsm + 2 * NPRIM * ss + t, ss, F, alfven);
     return;
   }
 #endif
   FT PL[NPRIM], PR[NPRIM];
-#pragma unroll
-  for (int s = 0; s < NPRIM; ++s) {
-    FT up = 0, lo = 0;
-    if (d.pidx[s] >= 0 && active)
-      recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, k, j, c), 1, up, lo);
-    PL[s] = __shfl_up_sync(0xffffffffu, up, 1);
+  recon_row<OPT>(d, p, cell, lane, active, edge[threadIdx.x >> 5], [&](int s, FT up, FT lo) {
+    PL[s] = up;
     PR[s] = lo;
-  }
+  });
+#pragma unroll
+  for (int s = 0; s < NPRIM; ++s) PL[s] = __shfl_up_sync(0xffffffffu, PL[s], 1);
   if (lane == 0 || !active) return;
-  face_flux<MT, 1, OPT>(d, p, b, k, j, c, PL, PR, F, alfven);
+  FaceGeo fg;
+  face_geo<MT, 1>(d, p, b, k, j, c, fg);
+  face_flux<MT, 1, OPT>(d, p, fg, b, k, j, c, PL, PR, F, alfven);
 }
 
 // x2 / x3 faces: a thread marches over MARCH consecutive faces of one
@@ -1062,7 +1238,6 @@ __device__ __forceinline__ void flux_march_body(const Dims &d, const pangu_param
   const int b = slot_of(d, (int)div_fast(r, na, ar));
   const int a = a0 + (int)ar;
   const long long stride = DIR == 2 ? (long long)d.N1 : (long long)d.N1 * d.N2;
-  const bool use_mc = PGK_FLUX_MC(p);
   const int f0 = m0 + run * MARCH;
   const int f1 = min(f0 + MARCH - 1, m1);
 #if PGK_SPLIT_FACES
@@ -1078,25 +1253,19 @@ __device__ __forceinline__ void flux_march_body(const Dims &d, const pangu_param
     {
       const int c = f0 - 1;
       const int kk = DIR == 2 ? a : c, jj = DIR == 2 ? c : a;
-#pragma unroll
-      for (int s = 0; s < NPRIM; ++s) {
-        FT up = 0, lo;
-        if (d.pidx[s] >= 0)
-          recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, kk, jj, i), stride, up, lo);
-        carry[s * ss] = up;
-      }
+      recon_vars<OPT>(d, p, [&](int v) { return a_prim(d, P, b, v) + coff(d, kk, jj, i); }, stride,
+                      [&](int s, FT up, FT) { carry[s * ss] = up; });
     }
     for (int f = f0; f <= f1; ++f) {
       const int kk = DIR == 2 ? a : f, jj = DIR == 2 ? f : a;
-#pragma unroll
-      for (int s = 0; s < NPRIM; ++s) {
-        FT up = 0, lo = 0;
-        if (d.pidx[s] >= 0)
-          recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, kk, jj, i), stride, up, lo);
-        next[s * ss] = up;
-        lower[s * ss] = lo;
-      }
-      face_flux_split<MT, DIR, OPT>(d, p, b, kk, jj, i, carry, lower, left_u, ss, F, alfven);
+      recon_vars<OPT>(d, p, [&](int v) { return a_prim(d, P, b, v) + coff(d, kk, jj, i); }, stride,
+                      [&](int s, FT up, FT lo) {
+                        next[s * ss] = up;
+                        lower[s * ss] = lo;
+                      });
+      FaceGeo fg;
+      face_geo<MT, DIR>(d, p, b, kk, jj, i, fg);
+      face_flux_split<MT, DIR, OPT>(d, p, fg, b, kk, jj, i, carry, lower, left_u, ss, F, alfven);
       double *tmp = carry;
       carry = next;
       next = tmp;
@@ -1108,24 +1277,20 @@ __device__ __forceinline__ void flux_march_body(const Dims &d, const pangu_param
   {
     const int c = f0 - 1;
     const int kk = DIR == 2 ? a : c, jj = DIR == 2 ? c : a;
-#pragma unroll
-    for (int s = 0; s < NPRIM; ++s) {
-      FT up = 0, lo;
-      if (d.pidx[s] >= 0) recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, kk, jj, i), stride, up, lo);
-      carry[s] = up;
-    }
+    recon_vars<OPT>(d, p, [&](int v) { return a_prim(d, P, b, v) + coff(d, kk, jj, i); }, stride,
+                    [&](int s, FT up, FT) { carry[s] = up; });
   }
   for (int f = f0; f <= f1; ++f) {
     const int kk = DIR == 2 ? a : f, jj = DIR == 2 ? f : a;
     FT PR[NPRIM], up[NPRIM];
-#pragma unroll
-    for (int s = 0; s < NPRIM; ++s) {
-      up[s] = 0.0;
-      PR[s] = 0.0;
-      if (d.pidx[s] >= 0)
-        recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, kk, jj, i), stride, up[s], PR[s]);
-    }
-    face_flux<MT, DIR, OPT>(d, p, b, kk, jj, i, carry, PR, F, alfven);
+    recon_vars<OPT>(d, p, [&](int v) { return a_prim(d, P, b, v) + coff(d, kk, jj, i); }, stride,
+                    [&](int s, FT u, FT lo) {
+                      up[s] = u;
+                      PR[s] = lo;
+                    });
+    FaceGeo fg;
+    face_geo<MT, DIR>(d, p, b, kk, jj, i, fg);
+    face_flux<MT, DIR, OPT>(d, p, fg, b, kk, jj, i, carry, PR, F, alfven);
 #pragma unroll
     for (int s = 0; s < NPRIM; ++s) carry[s] = up[s];
   }
@@ -1157,25 +1322,24 @@ __device__ __forceinline__ void flux_tile_body(const Dims &d, const pangu_params
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const int i = i0 + (int)ti * 32 + lane;
   const long long stride = DIR == 2 ? (long long)d.N1 : (long long)d.N1 * d.N2;
-  const bool use_mc = PGK_FLUX_MC(p);
   // cells mt0 - 1 .. mt0 + TF - 1: the lower neighbour of every face of the tile
   for (int cr = row; cr <= TF; cr += TF) {
     const int c = mt0 - 1 + cr;
     if (i <= i1 && c <= m1) {
       const int kk = DIR == 2 ? a : c, jj = DIR == 2 ? c : a;
-#pragma unroll
-      for (int s = 0; s < NPRIM; ++s) {
-        FT up = 0, lo = 0;
-        if (d.pidx[s] >= 0) recon_cell(use_mc, a_prim(d, P, b, d.pidx[s]) + coff(d, kk, jj, i), stride, up, lo);
-        sup[cr][s][lane] = up;
-        slo[cr][s][lane] = lo;
-      }
+      recon_vars<OPT>(d, p, [&](int v) { return a_prim(d, P, b, v) + coff(d, kk, jj, i); }, stride,
+                      [&](int s, FT up, FT lo) {
+                        sup[cr][s][lane] = up;
+                        slo[cr][s][lane] = lo;
+                      });
     }
   }
   __syncthreads();
   const int f = mt0 + row;
   if (i > i1 || f > m1) return;
   const int kk = DIR == 2 ? a : f, jj = DIR == 2 ? f : a;
+  FaceGeo fg;
+  face_geo<MT, DIR>(d, p, b, kk, jj, i, fg);
 #if PGK_SPLIT_FACES
   // sup[row][.][lane] and slo[row + 1][.][lane] are read by this thread only.
   // Tiles of 8 rows keep both states in registers (their static shared
@@ -1183,7 +1347,7 @@ __device__ __forceinline__ void flux_tile_body(const Dims &d, const pangu_params
   constexpr bool split = split_faces(MT) && TF <= 4;
   __shared__ double sul[split ? TF : 1][NPRIM][32];
   if (split) {
-    face_flux_split<MT, DIR, OPT>(d, p, b, kk, jj, i, &sup[row][0][lane], &slo[row + 1][0][lane],
+    face_flux_split<MT, DIR, OPT>(d, p, fg, b, kk, jj, i, &sup[row][0][lane], &slo[row + 1][0][lane],
                              &sul[split ? row : 0][0][lane], 32, F, alfven);
     return;
   }
@@ -1194,11 +1358,11 @@ __device__ __forceinline__ void flux_tile_body(const Dims &d, const pangu_params
     PL[s] = sup[row][s][lane];
     PR[s] = slo[row + 1][s][lane];
   }
-  face_flux<MT, DIR, OPT>(d, p, b, kk, jj, i, PL, PR, F, alfven);
+  face_flux<MT, DIR, OPT>(d, p, fg, b, kk, jj, i, PL, PR, F, alfven);
 }
 
 template <int MT, int DIR, int TF, int OPT>
-__global__ void __launch_bounds__(32 * TF, TF == 4 ? flux_blocks(MT) : 2) k_flux_tile(Dims d, pangu_params p, int k0,
+__global__ void __launch_bounds__(32 * TF, TF == 4 ? kFluxBlocks : 2) k_flux_tile(Dims d, pangu_params p, int k0,
                                                                      int k1, int j0, int j1, int i0,
                                                                      int i1, const PT *P, double *F,
                                                                      double *alfven) {
@@ -1273,16 +1437,23 @@ __device__ __forceinline__ bool tma_wait(unsigned long long *bar, int *err) {
 // two cells of its face.
 constexpr int kTmaCols = 32 + kTmaAlign;
 
+// Bytes of the staged primitives.
+template <int TF>
+__host__ __device__ inline size_t tma_tile_staged(int nf) {
+  return (size_t)nf * (TF + 5) * kTmaCols * sizeof(PT);
+}
 template <int TF>
 inline size_t tma_tile_smem(int nf) {
-  // the staged primitives, whose space then holds the split faces' states
-  const size_t staged = (size_t)nf * (TF + 5) * kTmaCols * sizeof(PT);
+  // the staged primitives and (FP64) the TF + 2 face values of each column, a
+  // space that then holds the split faces' states
+  const size_t staged = tma_tile_staged<TF>(nf) +
+                        (PGK_MIXED ? 0 : (size_t)nf * (TF + 2) * 32 * sizeof(double));
   const size_t split = split_faces(MKS) ? 3 * (size_t)TF * NPRIM * 32 * sizeof(double) : 0;
   return std::max(staged, split);
 }
 
 template <int MT, int DIR, int TF, int OPT>
-__global__ void __launch_bounds__(32 * TF, flux_blocks(MT))
+__global__ void __launch_bounds__(32 * TF, kFluxBlocks)
     k_flux_tile_tma(const __grid_constant__ CUtensorMap tm, Dims d, pangu_params p, int k0,
                     int k1, int j0, int j1, int i0, int i1, double *F, double *alfven,
                     int *err) {
@@ -1316,26 +1487,80 @@ __global__ void __launch_bounds__(32 * TF, flux_blocks(MT))
     else
       tma_load_4d(raw, &tm, xs, a, mt0 - 3, b * d.NF, &bar);
   }
-  if (!tma_wait(&bar, err)) return;
   const int i = x0 + lane, f = mt0 + row;
   const bool active = i <= i1 && f <= m1;
-  const bool use_mc = PGK_FLUX_MC(p);
+  const int kk = DIR == 2 ? a : f, jj = DIR == 2 ? f : a;
+  if (!tma_wait(&bar, err)) return;
   FT PL[NPRIM], PR[NPRIM];
 #pragma unroll
-  for (int s = 0; s < NPRIM; ++s) {
-    PL[s] = 0;
-    PR[s] = 0;
-    if (active && d.pidx[s] >= 0) {
-      // cell f - 1 sits at tile row row + 2, cell f at row + 3
-      const PT *q = raw + ((size_t)d.pidx[s] * R + row + 2) * kTmaCols + lane + off;
-      FT lo, up;
-      recon_cell(use_mc, q, kTmaCols, PL[s], lo);
-      recon_cell(use_mc, q + kTmaCols, kTmaCols, up, PR[s]);
+  for (int s = 0; s < NPRIM; ++s) PL[s] = PR[s] = 0;
+#if !PGK_MIXED
+  if (!(OPT & kFluxMC)) {
+    // The face values of the tile's columns, once each: face value r lies
+    // between the tile's rows r + 1 and r + 2, and (r, component) is a task of
+    // one warp. Then every thread limits the two cells of its face (rows
+    // row + 2 and row + 3).
+    FT *fv = reinterpret_cast<FT *>(dsm + tma_tile_staged<TF>(d.NF)) + lane;
+    unsigned redo = 0;  // tasks outside ppm4_face's range
+    // component v's TF + 2 values: one for each warp, and two more for two of
+    // them in turn
+    static_assert(TF == 4, "the tasks are laid out for four warps");
+#pragma unroll
+    for (int v = 0; v < NPRIM; ++v) {
+      const int r = (row + 2 * (v & 1)) & 3;
+      if (v < d.NF) {
+        const PT *q = raw + (v * R + r) * kTmaCols + lane + off;
+        bool ok = true;
+        fv[(v * (TF + 2) + r) * 32] =
+            ppm4_face(q[0], q[kTmaCols], q[2 * kTmaCols], q[3 * kTmaCols], ok);
+        if (!ok) redo |= 1u << (2 * v);
+        if (r < 2) {
+          q += 4 * kTmaCols;
+          ok = true;
+          fv[(v * (TF + 2) + r + 4) * 32] =
+              ppm4_face(q[0], q[kTmaCols], q[2 * kTmaCols], q[3 * kTmaCols], ok);
+          if (!ok) redo |= 2u << (2 * v);
+        }
+      }
     }
+    while (redo) {
+      const int t = __ffs(redo) - 1, v = t >> 1;
+      redo &= redo - 1;
+      const int r = ((row + 2 * (v & 1)) & 3) + 4 * (t & 1);
+      const PT *q = raw + (v * R + r) * kTmaCols + lane + off;
+      fv[(v * (TF + 2) + r) * 32] =
+          ppm4_face_plain(q[0], q[kTmaCols], q[2 * kTmaCols], q[3 * kTmaCols]);
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll
+      for (int s = 0; s < NPRIM; ++s)
+        if (d.pidx[s] >= 0) {
+          const int v = d.pidx[s];
+          const PT *q = raw + (v * R + row + 2) * kTmaCols + lane + off;
+          const FT *f3 = fv + (v * (TF + 2) + row) * 32;
+          const double fc = f3[32];
+          PL[s] = ppm4_side(q[0], f3[0], fc);
+          PR[s] = ppm4_side(q[kTmaCols], f3[64], fc);
+        }
+    }
+  } else
+#endif
+  if (active) {
+#pragma unroll
+    for (int s = 0; s < NPRIM; ++s)
+      if (d.pidx[s] >= 0) {
+        // cell f - 1 sits at tile row row + 2, cell f at row + 3
+        const PT *q = raw + ((size_t)d.pidx[s] * R + row + 2) * kTmaCols + lane + off;
+        FT lo, up;
+        recon_cell(PGK_FLUX_MC(p), q, kTmaCols, PL[s], lo);
+        recon_cell(PGK_FLUX_MC(p), q + kTmaCols, kTmaCols, up, PR[s]);
+      }
   }
   __syncthreads();  // the staged tile is read; its space is reused below
   if (!active) return;
-  const int kk = DIR == 2 ? a : f, jj = DIR == 2 ? f : a;
+  FaceGeo fg;
+  face_geo<MT, DIR>(d, p, b, kk, jj, i, fg);
 #if PGK_SPLIT_FACES
   if (split_faces(MT)) {
     double *sl = reinterpret_cast<double *>(dsm);
@@ -1347,11 +1572,11 @@ __global__ void __launch_bounds__(32 * TF, flux_blocks(MT))
       pl[s * 32] = PL[s];
       pr[s * 32] = PR[s];
     }
-    face_flux_split<MT, DIR, OPT>(d, p, b, kk, jj, i, pl, pr, ul, 32, F, alfven);
+    face_flux_split<MT, DIR, OPT>(d, p, fg, b, kk, jj, i, pl, pr, ul, 32, F, alfven);
     return;
   }
 #endif
-  face_flux<MT, DIR, OPT>(d, p, b, kk, jj, i, PL, PR, F, alfven);
+  face_flux<MT, DIR, OPT>(d, p, fg, b, kk, jj, i, PL, PR, F, alfven);
 }
 
 // x1 faces: a CTA of 4 warps takes 4 consecutive rows (j) of one k and one
@@ -1363,15 +1588,16 @@ constexpr int kTmaRowsX1 = 4;
 constexpr int kTmaColsX1 = (kFacesPerWarp + 5 + kTmaAlign - 1 + kTmaAlign - 1) / kTmaAlign *
                            kTmaAlign;
 
-inline size_t tma_x1_smem(int nf) {
-  const size_t staged = (size_t)nf * kTmaRowsX1 * kTmaColsX1 * sizeof(PT);
-  const size_t split = split_faces(MKS) ? 3 * (size_t)NPRIM * 32 * kTmaRowsX1 * sizeof(double)
-                                        : 0;
-  return std::max(staged, split);
+__host__ __device__ inline size_t tma_x1_staged(int nf) {
+  return (size_t)nf * kTmaRowsX1 * kTmaColsX1 * sizeof(PT);
+}
+inline size_t tma_x1_smem(int nf, bool split) {
+  return tma_x1_staged(nf) +
+         (split ? 3 * (size_t)NPRIM * 32 * kTmaRowsX1 * sizeof(double) : 0);
 }
 
 template <int MT, int OPT>
-__global__ void __launch_bounds__(32 * kTmaRowsX1, flux_blocks(MT))
+__global__ void __launch_bounds__(32 * kTmaRowsX1, kFluxBlocks)
     k_flux_x1_tma(const __grid_constant__ CUtensorMap tm, Dims d, pangu_params p, int k0, int k1,
                   int j0, int j1, int i0, int i1, double *F, double *alfven, int *err) {
   extern __shared__ __align__(128) unsigned char dsm[];
@@ -1399,46 +1625,46 @@ __global__ void __launch_bounds__(32 * kTmaRowsX1, flux_blocks(MT))
     mbar_expect_tx(&bar, (unsigned)(d.NF * kTmaRowsX1 * kTmaColsX1 * sizeof(PT)));
     tma_load_4d(raw, &tm, xs, jr0, k, b * d.NF, &bar);
   }
-  if (!tma_wait(&bar, err)) return;
   const int j = jr0 + w, c = c0 + lane;
   const bool active = c <= i1 && j <= j1;  // cell c is needed by face c (and c + 1)
-  const bool use_mc = PGK_FLUX_MC(p);
-  FT up[NPRIM], lo[NPRIM];
-#pragma unroll
-  for (int s = 0; s < NPRIM; ++s) {
-    up[s] = 0;
-    lo[s] = 0;
-    if (d.pidx[s] >= 0 && active)
-      recon_cell(use_mc, raw + ((size_t)d.pidx[s] * kTmaRowsX1 + w) * kTmaColsX1 + off + lane, 1,
-                 up[s], lo[s]);
-  }
+  __shared__ FT edge[kTmaRowsX1][NPRIM];
+  if (!tma_wait(&bar, err)) return;
+  auto cell = [&](int v, int l) {
+    return raw + (v * kTmaRowsX1 + w) * kTmaColsX1 + off + l;
+  };
 #if PGK_SPLIT_FACES
   if (split_faces(MT)) {
-    __syncthreads();  // the staged rows are read; their space is reused below
-    // [3][NPRIM][blockDim.x] as in k_flux_x1
-    double *fsm = reinterpret_cast<double *>(dsm);
+    // [3][NPRIM][blockDim.x] as in k_flux_x1, behind the staged rows
+    double *fsm = reinterpret_cast<double *>(dsm + tma_x1_staged(d.NF));
     const int ss = blockDim.x, t = threadIdx.x;
-#pragma unroll
-    for (int s = 0; s < NPRIM; ++s) {
-      fsm[s * ss + t] = up[s];
-      fsm[(NPRIM + s) * ss + t] = lo[s];
-    }
+    recon_row<OPT>(d, p, cell, lane, active, edge[w], [&](int s, FT u, FT l) {
+      fsm[s * ss + t] = u;
+      fsm[(NPRIM + s) * ss + t] = l;
+    });
     __syncwarp();
     if (lane == 0 || !active) return;
-    face_flux_split<MT, 1, OPT>(d, p, b, k, j, c, fsm + t - 1, fsm + NPRIM * ss + t,
+    FaceGeo fg;
+    face_geo<MT, 1>(d, p, b, k, j, c, fg);
+    face_flux_split<MT, 1, OPT>(d, p, fg, b, k, j, c, fsm + t - 1, fsm + NPRIM * ss + t,
                                 fsm + 2 * NPRIM * ss + t, ss, F, alfven);
     return;
   }
 #endif
-  FT PL[NPRIM];
+  FT PL[NPRIM], lo[NPRIM];
+  recon_row<OPT>(d, p, cell, lane, active, edge[w], [&](int s, FT u, FT l) {
+    PL[s] = u;
+    lo[s] = l;
+  });
 #pragma unroll
-  for (int s = 0; s < NPRIM; ++s) PL[s] = __shfl_up_sync(0xffffffffu, up[s], 1);
+  for (int s = 0; s < NPRIM; ++s) PL[s] = __shfl_up_sync(0xffffffffu, PL[s], 1);
   if (lane == 0 || !active) return;
-  face_flux<MT, 1, OPT>(d, p, b, k, j, c, PL, lo, F, alfven);
+  FaceGeo fg;
+  face_geo<MT, 1>(d, p, b, k, j, c, fg);
+  face_flux<MT, 1, OPT>(d, p, fg, b, k, j, c, PL, lo, F, alfven);
 }
 
 template <int MT, int MARCH, int OPT>
-__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT)) k_flux_march2(Dims d, pangu_params p, int k0, int k1,
+__global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_march2(Dims d, pangu_params p, int k0, int k1,
                                                           int j0, int j1, int i0, int i1,
                                                           const PT *P, double *F,
                                                           double *alfven) {
@@ -1446,7 +1672,7 @@ __global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT)) k_flux_march2(D
   flux_march_body<MT, 2, MARCH, OPT>(d, p, k0, k1, j0, j1, i0, i1, P, F, alfven);
 }
 template <int MT, int MARCH, int OPT>
-__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT)) k_flux_march3(Dims d, pangu_params p, int k0, int k1,
+__global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_march3(Dims d, pangu_params p, int k0, int k1,
                                                           int j0, int j1, int i0, int i1,
                                                           const PT *P, double *F,
                                                           double *alfven) {
@@ -2856,7 +3082,7 @@ void launch_flux_dir(const pangu_engine *e, const pangu_pack *md, int dir, int m
     const long long nt = (long long)d.NB * (k1 - k0 + 1) *
                          ((j1 - j0 + 1 + kTmaRowsX1 - 1) / kTmaRowsX1) * nseg;
     launch_pdl_smem(k_flux_x1_tma<MT, OPT>, dim3((unsigned)nt), dim3(32 * kTmaRowsX1),
-                    tma_x1_smem(d.NF), s, tm, d, e->p, k0, k1, j0, j1, i0, i1, F, md->alfven,
+                    tma_x1_smem(d.NF, split_faces(MT)), s, tm, d, e->p, k0, k1, j0, j1, i0, i1, F, md->alfven,
                     e->d_err);
     return;
   }

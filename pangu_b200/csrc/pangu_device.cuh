@@ -12,6 +12,7 @@
 
 #include <cstdint>
 
+#include "exactdiv.h"
 #include "pgmath.h"
 
 // Powers, exponentials and logarithms: correctly rounded (pgmath.h) in the
@@ -478,20 +479,141 @@ PGD void fast_speed_from_state(double gam, const double P[NPRIM], const Geo &g, 
   }
 }
 
+// Plain division out of line: the fallback for single quotients that the
+// branch-free forms refuse, kept out of the kernels' instruction stream.
+__device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+
+// calc_state and fast_speed_from_state with their eight divisions by xd::quot
+// (al: the reciprocal of the lapse): the same values while every operand is in
+// range, which the return value says; else the caller uses the plain forms.
+template <int MT>
+PGD bool state_speed(double gam, const double P[NPRIM], const Geo &g, const xd::Rcp &al, int dir,
+                     State &s, double &vmax, double &vmin) {
+  constexpr Pattern PT = metric_pattern(MT);
+  const double alpha = g.alpha;
+  const double u[3] = {P[UX1], P[UX2], P[UX3]};
+  double sq = 0.0;
+#pragma unroll
+  for (int i = 1; i < 4; ++i)
+#pragma unroll
+    for (int j = 1; j < 4; ++j)
+      if (PT.nz[i][j]) sq = sq + u[i - 1] * g.gcov[i][j] * u[j - 1];
+  const double lor = sqrt(1.0 + sq);
+  bool ok = xd::in_range(lor);
+  s.ucon[0] = MT == MINKOWSKI ? lor : xd::quot(lor, al);
+#pragma unroll
+  for (int i = 1; i < 4; ++i)
+    s.ucon[i] = PT.nz[0][i] ? u[i - 1] - s.ucon[0] * g.gcon[0][i] * alpha * alpha : u[i - 1];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    double v = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (PT.nz[r][c]) v += g.gcov[r][c] * s.ucon[c];
+    s.ucov[r] = v;
+  }
+  s.bcon[0] = P[BX1] * s.ucov[1] + P[BX2] * s.ucov[2] + P[BX3] * s.ucov[3];
+  ok &= xd::in_range_den(s.ucon[0]);
+  const xd::Rcp iu = xd::rcp(s.ucon[0]);
+  double n[3];
+  bool bok = true;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    n[i] = P[BX1 + i] + s.bcon[0] * s.ucon[i + 1];
+    bok &= xd::in_range0(n[i]);
+    s.bcon[i + 1] = xd::quot_s(n[i], iu);
+  }
+  // a field that spreads into a field-free gas is that small at its front
+  if (!bok)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s.bcon[i + 1] = div_plain(n[i], s.ucon[0]);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    double v = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (PT.nz[r][c]) v += g.gcov[r][c] * s.bcon[c];
+    s.bcov[r] = v;
+  }
+  s.bsq = s.bcon[0] * s.bcov[0] + s.bcon[1] * s.bcov[1] + s.bcon[2] * s.bcov[2] +
+          s.bcon[3] * s.bcov[3];
+  const double hh = P[RHO] + gam * P[ENY];
+  const double h_tot = s.bsq + hh;
+  const double cs_n = gam * (gam - 1.) * P[ENY];
+  // b^2 may be any small number: cs_sq >= 2^-360 absorbs a va_sq whose last bits
+  // an underflow would change (below 2^-560)
+  ok &= xd::in_range_den(hh) & xd::in_range_den(h_tot) & xd::below(s.bsq, 400) &
+        xd::below(cs_n, 400) & !xd::below(cs_n, -300);
+  const double va_sq = xd::quot(s.bsq, xd::rcp(h_tot));
+  const double cs_sq = xd::quot(cs_n, xd::rcp(hh));
+  double cf_sq = cs_sq + va_sq - cs_sq * va_sq;
+  if (cf_sq < 0.) cf_sq = 1e-10;
+  if (cf_sq > 1.) cf_sq = 1.;
+  const double n_sq = g.gcon[dir][dir];
+  const double t_sq = g.gcon[0][0];
+  const double n_dot_t = g.gcon[0][dir];
+  const double nu2 = s.ucon[dir] * s.ucon[dir];
+  const double tu2 = s.ucon[0] * s.ucon[0];
+  const double nutu = s.ucon[dir] * s.ucon[0];
+  const double A = tu2 - (t_sq + tu2) * cf_sq;
+  const double B = 2. * (nutu - (n_dot_t + nutu) * cf_sq);
+  const double C = nu2 - (n_sq + nu2) * cf_sq;
+  double disc = B * B - 4. * A * C;
+  if (disc < 0.0 && disc != -1.e-10) disc = 0.0;
+  disc = sqrt(disc);
+  const double A2 = 2. * A;
+  const double np = -(-B + disc), nm = -(-B - disc);
+  ok &= xd::in_range_den(A2) & xd::in_range0(np) & xd::in_range0(nm);
+  const xd::Rcp ia = xd::rcp(A2);
+  const double vp = xd::quot(np, ia);
+  const double vm = xd::quot(nm, ia);
+  const bool pm = vp > vm;
+  vmax = pm ? vp : vm;
+  vmin = pm ? vm : vp;
+  return ok;
+}
+
 // ---------------------------------------------------------------------------
 // interpolation/ (interpolater_mc.h:16-48, interpolater_ppm4.h:29-67)
 // ---------------------------------------------------------------------------
-PGD double minmod3(double a, double b, double c) {
-  if (a > 0.0 && b > 0.0 && c > 0.0) return fmin(fmin(a, b), c);
-  if (a < 0.0 && b < 0.0 && c < 0.0) return fmax(fmax(a, b), c);
-  return 0.0;
-}
 // Right value at the upper face (ql_ip1) and left value at the lower face
 // (qr_i) of the centre cell of a 3-point MC stencil.
+// The slope is minmod(a, b, c) with a = 2 (q - qm1), c = 2 (qp1 - q) and their
+// mean b. Where a and c have one sign so has b, and the smallest magnitude of
+// the three is the answer (0 when one of them is 0, so the signs' bits decide);
+// a NaN neighbour makes b, hence m, NaN and the slope 0.
 PGD void mc(double qm1, double q, double qp1, double &ql_ip1, double &qr_i) {
-  const double slope = minmod3(2.0 * (q - qm1), 0.5 * (qp1 - qm1), 2.0 * (qp1 - q));
+  const double a = 2.0 * (q - qm1), b = 0.5 * (qp1 - qm1), c = 2.0 * (qp1 - q);
+  double m = fabs(a) < fabs(c) ? a : c;
+  m = fabs(m) <= fabs(b) ? m : b;
+  const bool same = (int)(xd::hi_bits(a) ^ xd::hi_bits(c)) >= 0;
+  const double slope = same && m == m ? m : 0.0;
   ql_ip1 = q + 0.5 * slope;
   qr_i = q - 0.5 * slope;
+}
+// PPM4 in two parts, so that the value at a face is formed once for its two
+// cells: the interpolant and its clamping between the adjacent cell values are
+// the same sums and comparisons seen from either cell. ppm4_face clears ok
+// where the stencil is not finite or the numerator too small for xd::div12; the
+// caller then uses ppm4 (or ppm4_face_plain) for that variable. Finite operands need no NaN rules, so the clamps are
+// plain compares and selects (a zero may keep the other sign).
+PGD double ppm4_face(double qm1, double q, double qp1, double qp2, bool &ok) {
+  const double n = 7.0 * (q + qp1) - (qm1 + qp2);
+  ok &= xd::in_range0(n);
+  const double v = xd::div12(n);
+  // below both, above both (then the nearer of them), or between
+  const bool b0 = v < q, b1 = v < qp1;
+  const double end = (b0 == (q < qp1)) ? q : qp1;
+  return b0 == b1 ? end : v;
+}
+// Upper-face value of a cell from its clamped face values; the lower-face
+// value is ppm4_side(q, up, lo). 2 x is exact, so q - 2 x is one rounding, and
+// the sign of |qc| - 2 |qd| rounded is the comparison's.
+PGD double ppm4_side(double q, double lo, double up) {
+  const double qc = up - q, qd = lo - q;
+  const bool far = (int)xd::hi_bits(__fma_rn(-2.0, fabs(qd), fabs(qc))) >= 0;
+  const double steep = far ? __fma_rn(-2.0, qd, q) : up;
+  return (qc * qd) >= 0.0 ? q : steep;
 }
 PGD void ppm4(double qm2, double qm1, double q, double qp1, double qp2, double &ql_ip1,
               double &qr_i) {
@@ -1044,6 +1166,24 @@ PGD double clamp_by_ratio(double rmin, double rmax, double total, double electro
   const double hi = total / (1.0 + rmin);
   const double b = kmax(0.0, kmin(electron, total));
   return kmax(lo, kmin(b, hi));
+}
+
+// Out-of-line forms for operands that the branch-free ones above refuse, kept
+// out of the instruction stream of the kernels' ordinary path.
+template <int MT>
+__device__ __noinline__ void side_plain(double gam, const double *P, const Geo *g, int dir,
+                                        State *s, double *v) {
+  calc_state<MT>(P, *g, *s);
+  fast_speed_from_state(gam, P, *g, *s, dir, v[0], v[1]);
+}
+__device__ __noinline__ double ppm4_face_plain(double qm1, double q, double qp1, double qp2) {
+  const double v = (7.0 * (q + qp1) - (qm1 + qp2)) / 12.0;
+  return fmin(fmax(v, fmin(q, qp1)), fmax(q, qp1));
+}
+__device__ __noinline__ double2 ppm4_plain(const double *q, long long st) {
+  double2 r;
+  ppm4(q[-2 * st], q[-st], q[0], q[st], q[2 * st], r.x, r.y);
+  return r;
 }
 
 // ---------------------------------------------------------------------------
