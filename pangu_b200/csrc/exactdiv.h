@@ -109,23 +109,28 @@ struct Rcp {
   double nb, y, yl;  // -b, RN(1/b), and y (1 - b y)
 };
 
-// From a first approximation y0 of 1/b (|1 - b y0| < 2^-19).
-XD_FN Rcp rcp_from(double b, double y0) {
-  const double nb = -b;
-  double e = fma_(nb, y0, 1.0);
+// RN(1/b) for an in-range denominator, from a first approximation y0 of 1/b
+// (|1 - b y0| < 2^-19).
+XD_FN double recip_from(double b, double y0) {
+  double e = fma_(-b, y0, 1.0);
   e = fma_(e, e, e);
   double y = fma_(y0, e, y0);
-  e = fma_(nb, y, 1.0);
-  y = fma_(y, e, y);
-  return {nb, y, mul_(y, fma_(nb, y, 1.0))};
+  e = fma_(-b, y, 1.0);
+  return fma_(y, e, y);
+}
+XD_FN Rcp rcp_from(double b, double y0) {
+  const double y = recip_from(b, y0);
+  return {-b, y, mul_(y, fma_(-b, y, 1.0))};
 }
 
 #if defined(__CUDACC__)
-__device__ __forceinline__ Rcp rcp(double b) {
+__device__ __forceinline__ double rcp_seed(double b) {
   double y0;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
-  return rcp_from(b, y0);
+  return y0;
 }
+__device__ __forceinline__ Rcp rcp(double b) { return rcp_from(b, rcp_seed(b)); }
+__device__ __forceinline__ double recip(double b) { return recip_from(b, rcp_seed(b)); }
 #endif
 
 // RN(a / b) for in-range operands.

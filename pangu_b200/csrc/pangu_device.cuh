@@ -483,12 +483,11 @@ PGD void fast_speed_from_state(double gam, const double P[NPRIM], const Geo &g, 
 // branch-free forms refuse, kept out of the kernels' instruction stream.
 __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
 
-// calc_state and fast_speed_from_state with their eight divisions by xd::quot
-// (al: the reciprocal of the lapse): the same values while every operand is in
-// range, which the return value says; else the caller uses the plain forms.
+// calc_state with its four divisions by xd::quot (al: the reciprocal of the
+// lapse): the same values while every operand is in range, which the return
+// value says; else the caller uses calc_state.
 template <int MT>
-PGD bool state_speed(double gam, const double P[NPRIM], const Geo &g, const xd::Rcp &al, int dir,
-                     State &s, double &vmax, double &vmin) {
+PGD bool state_part(const double P[NPRIM], const Geo &g, const xd::Rcp &al, State &s) {
   constexpr Pattern PT = metric_pattern(MT);
   const double alpha = g.alpha;
   const double u[3] = {P[UX1], P[UX2], P[UX3]};
@@ -537,6 +536,15 @@ PGD bool state_speed(double gam, const double P[NPRIM], const Geo &g, const xd::
   }
   s.bsq = s.bcon[0] * s.bcov[0] + s.bcon[1] * s.bcov[1] + s.bcon[2] * s.bcov[2] +
           s.bcon[3] * s.bcov[3];
+  return ok;
+}
+
+// State and signal speeds (calc_state and fast_speed_from_state) likewise: eight
+// divisions.
+template <int MT>
+PGD bool state_speed(double gam, const double P[NPRIM], const Geo &g, const xd::Rcp &al, int dir,
+                     State &s, double &vmax, double &vmin) {
+  bool ok = state_part<MT>(P, g, al, s);
   const double hh = P[RHO] + gam * P[ENY];
   const double h_tot = s.bsq + hh;
   const double cs_n = gam * (gam - 1.) * P[ENY];
@@ -643,6 +651,7 @@ PGD void ppm4(double qm2, double qm1, double q, double qp1, double qp2, double &
 constexpr int MAX_NEWT_ITER = 30;
 constexpr double NEWT_TOL = 1e-10;
 constexpr double MIN_NEWT_TOL = 1e-10;
+static_assert(NEWT_TOL == MIN_NEWT_TOL, "newton_2d_done tests one tolerance");
 constexpr int EXTRA_NEWT_ITER = 2;
 constexpr double W_TOO_BIG = 1.e20;
 constexpr double UTSQ_TOO_BIG = 1.e20;
@@ -711,10 +720,23 @@ PGD bool harm_utsq(const double prim[9], const Geo &g, double &utsq) {
 template <int MT>
 PGD void harm_velocity(const Harm &s, double Gamma, double W, double prim[9]) {
   constexpr Pattern PT = metric_pattern(MT);
+  const double fac = Gamma / (W + s.Bsq);
+  const xd::Rcp iw = xd::rcp(W);
+  double n[3], q[3];
+  bool ok = xd::in_range_den(W);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    n[i] = s.QdotB * s.Bcon[i + 1];
+    ok &= xd::in_range0(n[i]);
+    q[i] = xd::quot(n[i], iw);
+  }
+  if (!ok)
+#pragma unroll
+    for (int i = 0; i < 3; i++) q[i] = div_plain(n[i], W);
 #pragma unroll
   for (int i = 1; i < 4; i++) {
     const double qt = PT.nz[i][0] ? s.Qcon[i] + s.ncon[i] * s.Qdotn : s.Qcon[i];
-    prim[UX1 + i - 1] = Gamma / (W + s.Bsq) * (qt + s.QdotB * s.Bcon[i] / W);
+    prim[UX1 + i - 1] = fac * (qt + q[i - 1]);
   }
 }
 
@@ -726,6 +748,93 @@ PGD double vsq_calc(double Bsq, double QdotBsq, double Qtsq, double W) {
 
 PGD bool w_too_small(double W, double Bsq, double QdotBsq, double Qtsq) {
   return (W * W * W * (W + 2. * Bsq) - QdotBsq * (2. * W + Bsq)) <= W * W * (Qtsq - Bsq * Bsq);
+}
+
+// What a Newton step of Scheme2D reads besides (W, v^2).
+struct Newton2d {
+  double Bsq, QdotBsq, Qtsq, Qdotn, D, g;
+};
+
+// The step (func_vsq, scheme_2d.h:99-156) at (W, vsq), divided plainly:
+// o = {dW, dvsq, df}.
+__device__ __noinline__ void newton_2d_plain(const Newton2d *c, double W, double vsq, double *o) {
+  const double g = c->g, Bsq = c->Bsq, QdotBsq = c->QdotBsq, D = c->D;
+  const double Wsq = W * W;
+  const double gtmp = 1. - vsq;
+  const double sgt = sqrt(gtmp);
+  const double p_tmp = ((g - 1.) * (W * gtmp - D * sgt) / g);
+  const double dPdW = ((g - 1.) * (1. - vsq) / g);
+  const double dPdvsq = ((g - 1.) * (0.5 * D / sgt - W) / g);
+  const double t2 = -0.5 * Bsq + dPdvsq;
+  const double t3 = Bsq + W;
+  const double t4 = t3 * t3;
+  const double t9 = 1.0 / Wsq;
+  const double t11 = c->Qtsq - vsq * t4 + QdotBsq * (Bsq + 2.0 * W) * t9;
+  const double t16 = QdotBsq * t9;
+  const double t18 = -c->Qdotn - 0.5 * Bsq * (1.0 + vsq) + 0.5 * t16 - W + p_tmp;
+  const double t21 = 1.0 / t3;
+  const double t23 = 1.0 / W;
+  const double t24 = t16 * t23;
+  const double t25 = -1.0 + dPdW - t24;
+  const double t35 = t25 * t3 + (Bsq - 2.0 * dPdvsq) * (QdotBsq + vsq * Wsq * W) * t9 * t23;
+  const double t36 = 1.0 / t35;
+  o[0] = -(t2 * t11 + t4 * t18) * t21 * t36;
+  const double t40 = (vsq + t24) * t3;
+  o[1] = -(-t25 * t11 - 2.0 * t40 * t18) * t21 * t36;
+  o[2] = -t11 * t11 - t18 * t18;
+}
+// Whether the relative size of a step that led to (x0, x1) (scheme_2d.h:200-206)
+// is at most (bit 0) or above (bit 1) the tolerance. The size itself is used
+// for nothing else, so a quotient to 2^-19 decides unless it is that close to
+// the tolerance (or an operand is out of range): then it is formed exactly.
+__device__ __noinline__ int newton_2d_done_plain(double x0, double dx0, double x1, double dx1) {
+  double e = (x0 == 0.) ? fabs(dx0) : fabs(dx0 / x0);
+  e += (x1 == 0.) ? fabs(dx1) : fabs(dx1 / x1);
+  return (fabs(e) <= NEWT_TOL ? 1 : 0) | (fabs(e) > NEWT_TOL ? 2 : 0);
+}
+PGD int newton_2d_done(double x0, double dx0, double x1, double dx1) {
+  const double d1 = (x1 == 0.) ? 1.0 : x1;
+  const double e = fabs(dx0) * fabs(xd::rcp_seed(x0)) + fabs(dx1) * fabs(xd::rcp_seed(d1));
+  const bool in = xd::in_range_den(x0) & xd::in_range_den(d1);
+  if (in & (e < NEWT_TOL * (1.0 - 0x1p-17))) return 1;
+  if (in & (e > NEWT_TOL * (1.0 + 0x1p-17)) & (e < 1e300)) return 2;
+  return newton_2d_done_plain(x0, dx0, x1, dx1);
+}
+
+// The step with its nine divisions branch-free (exactdiv.h), the three by
+// gamma sharing the reciprocal rg; false where an operand is out of range.
+PGD bool newton_2d_step(const Newton2d &c, const xd::Rcp &rg, double W, double vsq, double &dx0,
+                        double &dx1, double &df) {
+  const double g = c.g, Bsq = c.Bsq, QdotBsq = c.QdotBsq, D = c.D;
+  const double Wsq = W * W;
+  const double gtmp = 1. - vsq;
+  const double sgt = sqrt(gtmp);
+  const double hD = 0.5 * D, t3 = Bsq + W;
+  const double t9 = xd::recip(Wsq), t21 = xd::recip(t3), t23 = xd::recip(W);
+  const double n1 = (g - 1.) * (W * gtmp - D * sgt);
+  const double n2 = (g - 1.) * (1. - vsq);
+  const double n3 = (g - 1.) * (xd::quot(hD, xd::rcp(sgt)) - W);
+  bool ok = xd::in_range(hD) & xd::in_range_den(sgt) & xd::in_range0(n1) & xd::in_range0(n2) &
+            xd::in_range0(n3) & xd::in_range_den(Wsq) & xd::in_range_den(t3) &
+            xd::in_range_den(W);
+  const double p_tmp = xd::quot(n1, rg);
+  const double dPdW = xd::quot(n2, rg);
+  const double dPdvsq = xd::quot(n3, rg);
+  const double t2 = -0.5 * Bsq + dPdvsq;
+  const double t4 = t3 * t3;
+  const double t11 = c.Qtsq - vsq * t4 + QdotBsq * (Bsq + 2.0 * W) * t9;
+  const double t16 = QdotBsq * t9;
+  const double t18 = -c.Qdotn - 0.5 * Bsq * (1.0 + vsq) + 0.5 * t16 - W + p_tmp;
+  const double t24 = t16 * t23;
+  const double t25 = -1.0 + dPdW - t24;
+  const double t35 = t25 * t3 + (Bsq - 2.0 * dPdvsq) * (QdotBsq + vsq * Wsq * W) * t9 * t23;
+  ok &= xd::in_range_den(t35);
+  const double t36 = xd::recip(t35);
+  dx0 = -(t2 * t11 + t4 * t18) * t21 * t36;
+  const double t40 = (vsq + t24) * t3;
+  dx1 = -(-t25 * t11 - 2.0 * t40 * t18) * t21 * t36;
+  df = -t11 * t11 - t18 * t18;
+  return ok;
 }
 
 // Scheme2D::invert (scheme_2d.h:257-404) with general_newton_raphson
@@ -749,62 +858,47 @@ PGD int invert_2d(const double U[9], double prim[9], double g, const Geo &geo,
     const double vsq = fabs(vsq_calc(s.Bsq, s.QdotBsq, s.Qtsq, W_last));
     x1 = (vsq > 1.) ? (1.0 - 1.e-15) : vsq;
   }
-  const double Bsq = s.Bsq, QdotBsq = s.QdotBsq, Qtsq = s.Qtsq, Qdotn = s.Qdotn, D = s.D;
-  const double gm1g = (g - 1.) / g;
-  double f = 1., df = 1., errx = 1.;
+  const Newton2d nc = {s.Bsq, s.QdotBsq, s.Qtsq, s.Qdotn, s.D, g};
+  const xd::Rcp rg = xd::rcp(g);
+  const bool g_ok = xd::in_range_den(g);
+  double f = 1., df = 1.;
+  int done = 2;
   int i_extra = 0, doing_extra = 0;
   for (int n_iter = 0;; ++n_iter) {
-    const double W = x0, vsq = x1;
-    const double Wsq = W * W;
-    const double gtmp = 1. - vsq;
-    const double sgt = sqrt(gtmp);
-    const double p_tmp = ((g - 1.) * (W * gtmp - D * sgt) / g);
-    const double dPdW = ((g - 1.) * (1. - vsq) / g);
-    const double dPdvsq = ((g - 1.) * (0.5 * D / sgt - W) / g);
-    (void)gm1g;
-    const double t2 = -0.5 * Bsq + dPdvsq;
-    const double t3 = Bsq + W;
-    const double t4 = t3 * t3;
-    const double t9 = 1.0 / Wsq;
-    const double t11 = Qtsq - vsq * t4 + QdotBsq * (Bsq + 2.0 * W) * t9;
-    const double t16 = QdotBsq * t9;
-    const double t18 = -Qdotn - 0.5 * Bsq * (1.0 + vsq) + 0.5 * t16 - W + p_tmp;
-    const double t21 = 1.0 / t3;
-    const double t23 = 1.0 / W;
-    const double t24 = t16 * t23;
-    const double t25 = -1.0 + dPdW - t24;
-    const double t35 = t25 * t3 + (Bsq - 2.0 * dPdvsq) * (QdotBsq + vsq * Wsq * W) * t9 * t23;
-    const double t36 = 1.0 / t35;
-    const double dx0 = -(t2 * t11 + t4 * t18) * t21 * t36;
-    const double t40 = (vsq + t24) * t3;
-    const double dx1 = -(-t25 * t11 - 2.0 * t40 * t18) * t21 * t36;
-    df = -t11 * t11 - t18 * t18;
+    double dx0, dx1;
+    if (!(newton_2d_step(nc, rg, x0, x1, dx0, dx1, df) & g_ok)) {
+      const Newton2d cc = nc;
+      double o[3];
+      newton_2d_plain(&cc, x0, x1, o);
+      dx0 = o[0];
+      dx1 = o[1];
+      df = o[2];
+    }
     f = -0.5 * df;
     const double xo0 = x0;
     x0 += dx0;
     x1 += dx1;
-    errx = (x0 == 0.) ? fabs(dx0) : fabs(dx0 / x0);
-    errx += (x1 == 0.) ? fabs(dx1) : fabs(dx1 / x1);
+    done = newton_2d_done(x0, dx0, x1, dx1);
     x0 = fabs(x0);
     x0 = (x0 > W_TOO_BIG) ? xo0 : x0;
     x1 = (x1 < 0.) ? 0. : x1;
     x1 = (x1 > 1.) ? (1. - 1.e-15) : x1;
-    if ((fabs(errx) <= NEWT_TOL) && (doing_extra == 0) && (EXTRA_NEWT_ITER > 0)) doing_extra = 1;
+    if ((done & 1) && (doing_extra == 0) && (EXTRA_NEWT_ITER > 0)) doing_extra = 1;
     if (doing_extra == 1) i_extra++;
-    if (((fabs(errx) <= NEWT_TOL) && (doing_extra == 0)) || (i_extra > EXTRA_NEWT_ITER) ||
+    if (((done & 1) && (doing_extra == 0)) || (i_extra > EXTRA_NEWT_ITER) ||
         (n_iter >= (MAX_NEWT_ITER - 1)))
       break;
   }
   int retval = 0;
   if (!isfinite(f) || !isfinite(df)) retval = 2;
-  else if (fabs(errx) > MIN_NEWT_TOL) retval = 1;
+  else if (done & 2) retval = 1;  // MIN_NEWT_TOL is NEWT_TOL
   const double W = x0, vsq = x1;
   if ((retval != 0) || (W == FAIL_VAL)) return retval * 100 + 1;
   if (W <= 0. || W > W_TOO_BIG) return 3;
   if (vsq >= 1.) return 4;
   const double gtmp = sqrt(1. - vsq);
   Gamma = 1. / gtmp;
-  rho0 = D * gtmp;
+  rho0 = s.D * gtmp;
   w = W * (1. - vsq);
   p = ((g - 1.) * (w - rho0) / g);
   uu = w - (rho0 + p);
