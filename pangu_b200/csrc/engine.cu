@@ -213,15 +213,15 @@ int pool_init(pangu_engine *e, int capacity, int max_jobs) {
   rc |= dalloc(&e->d_xsrc, (size_t)e->xch_cap);
   if (p.metric_type == PANGU_METRIC_MKS || p.metric_type == PANGU_METRIC_BL) {
     const TabLayout T = p.metric_type == PANGU_METRIC_MKS ? tab_layout(MKS) : tab_layout(BL);
-    const size_t pc = (size_t)d.N2 * d.N1, p1 = (size_t)d.N2 * (d.N1 + 1),
-                 p2 = (size_t)(d.N2 + 1) * d.N1;
-    rc |= dalloc(&e->d_ctab, (size_t)capacity * T.ncen * pc);
-    rc |= dalloc(&e->d_f1tab, (size_t)capacity * T.nmet * p1);
-    rc |= dalloc(&e->d_f2tab, (size_t)capacity * T.nmet * p2);
+    const size_t rows = (size_t)capacity * d.N2, rows2 = (size_t)capacity * (d.N2 + 1);
+    const size_t n1 = rows * tab_row(d.N1 + 1, T.nmet), n2 = rows2 * tab_row(d.N1, T.nmet);
+    rc |= dalloc(&e->d_ctab, rows * tab_row(d.N1, T.ncen));
+    rc |= dalloc(&e->d_f1tab, n1);
+    rc |= dalloc(&e->d_f2tab, n2);
     if (p.precision == PANGU_PRECISION_MIXED) {
-      rc |= dalloc(&e->d_ctab32, (size_t)capacity * T.nconn * pc);
-      rc |= dalloc(&e->d_f1tab32, (size_t)capacity * T.nmet * p1);
-      rc |= dalloc(&e->d_f2tab32, (size_t)capacity * T.nmet * p2);
+      rc |= dalloc(&e->d_ctab32, rows * tab_row(d.N1, T.ncen));
+      rc |= dalloc(&e->d_f1tab32, n1);
+      rc |= dalloc(&e->d_f2tab32, n2);
     }
   }
   if (rc != PANGU_OK) return PANGU_ENOMEM;
@@ -403,16 +403,11 @@ int pool_attach(pangu_engine *e, const pangu_mesh &m, double a, double h, int *j
         k_build_tables<BL><<<grid_for(n), kThreads>>>(dj, J.p, e->d_ctab, e->d_f1tab, e->d_f2tab);
       if (e->d_ctab32) {
         const TabLayout T = e->p.metric_type == PANGU_METRIC_MKS ? tab_layout(MKS) : tab_layout(BL);
-        const long long nc = (long long)dj.NB * T.nconn * d.N2 * d.N1;
-        if (e->p.metric_type == PANGU_METRIC_MKS)
-          k_conn_to_f32<MKS><<<grid_for(nc), kThreads>>>(dj, e->d_ctab32);
-        else
-          k_conn_to_f32<BL><<<grid_for(nc), kThreads>>>(dj, e->d_ctab32);
-        const long long p1 = (long long)d.N2 * (d.N1 + 1), p2 = (long long)(d.N2 + 1) * d.N1;
-        k_planes_to_f32<<<grid_for((long long)dj.NB * T.nmet * p1), kThreads>>>(
-            dj, e->d_f1tab, e->d_f1tab32, T.nmet, p1);
-        k_planes_to_f32<<<grid_for((long long)dj.NB * T.nmet * p2), kThreads>>>(
-            dj, e->d_f2tab, e->d_f2tab32, T.nmet, p2);
+        const long long nc = d.N2 * tab_row(d.N1, T.ncen);
+        k_table_to_f32<<<grid_for(dj.NB * nc), kThreads>>>(dj, e->d_ctab, e->d_ctab32, nc);
+        const long long n1 = d.N2 * tab_row(d.N1 + 1, T.nmet), n2 = (d.N2 + 1) * tab_row(d.N1, T.nmet);
+        k_table_to_f32<<<grid_for(dj.NB * n1), kThreads>>>(dj, e->d_f1tab, e->d_f1tab32, n1);
+        k_table_to_f32<<<grid_for(dj.NB * n2), kThreads>>>(dj, e->d_f2tab, e->d_f2tab32, n2);
       }
       ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
     }

@@ -57,11 +57,12 @@ struct Dims {
   const double *t2;      // [slot][12][N2 + 1]
   const double *origin;  // [slot][3]
   // Static MKS/BL metric tables (built once per engine by k_build_tables):
-  // component planes of [NB][comp][N2][N1] (centres), [NB][comp][N2][N1+1]
-  // (x1 faces) and [NB][comp][N2+1][N1] (x2 faces); x3 faces use the centres.
+  // N2 x N1 points per slot at the centres, N2 x (N1 + 1) at the x1 faces and
+  // (N2 + 1) x N1 at the x2 faces, laid out by tab_at (kernels.cuh); x3 faces use
+  // the centres.
   const double *ctab, *f1tab, *f2tab;
-  // Mixed form only: the centre table's Christoffel planes rounded once to
-  // FP32, [slot][nconn][N2][N1], read by the FP32 source term; null otherwise.
+  // Mixed form only: the centre table rounded once to FP32, read by the FP32
+  // source term, electron heating and the x3 faces; null otherwise.
   const float *ctab32;
   // Mixed form only: the x1- and x2-face tables rounded once to FP32 (the
   // FP32 face fluxes read these); null otherwise.
@@ -109,7 +110,7 @@ struct pangu_engine {
   signed char *d_bcf = nullptr; // [capacity][6]
   double *d_t1 = nullptr, *d_t2 = nullptr, *d_origin = nullptr;
   double *d_ctab = nullptr, *d_f1tab = nullptr, *d_f2tab = nullptr;
-  float *d_ctab32 = nullptr;  // mixed form: FP32 Christoffel planes
+  float *d_ctab32 = nullptr;  // mixed form: FP32 centre table
   float *d_f1tab32 = nullptr, *d_f2tab32 = nullptr;  // mixed form: FP32 face tables
   long long *d_xdst = nullptr, *d_xsrc = nullptr;  // [capacity x ghost cells per block]
   long long nxch = 0, xch_cap = 0;

@@ -59,6 +59,7 @@ __host__ __forceinline__ PT *prim_of(const Pack *md) {
 // one wave (1.2 % per cycle; at 64 registers its Newton loop spills too much).
 constexpr int kThreads = 256;
 constexpr int kRecoveryThreads = 128;
+constexpr int kFixThreads = 128;
 
 // Programmatic dependent launch: the stage's kernels are launched with
 // programmatic stream serialisation (launch_pdl), so the launch of a kernel
@@ -255,15 +256,30 @@ __host__ __device__ constexpr TabLayout tab_layout(int mt) {
   return L;
 }
 
+// A table holds its nc components of the points (j, i) of a slot as
+// [slot][j][i / kTabCols][component][i % kTabCols]: the components of one point
+// lie a constant 128 bytes apart, so that a thread forms one address and every
+// load takes its component as an immediate offset (a plane per component cost
+// two or three integer instructions a load), and a warp's 32 columns read whole
+// 128-byte lines as before.
+constexpr int kTabCols = 16;
+__host__ __device__ constexpr long long tab_row(int W, int nc) {
+  return (long long)((W + kTabCols - 1) / kTabCols) * kTabCols * nc;
+}
+// Offset of component 0 of point (j, i) of slot b (rows of W points, R rows).
+__device__ __forceinline__ long long tab_at(int nc, int R, int W, int b, int j, int i) {
+  return ((long long)b * R + j) * tab_row(W, nc) +
+         (unsigned)(i / kTabCols * kTabCols * nc + i % kTabCols);
+}
+
 template <int MT>
-__device__ __forceinline__ int load_geo(const double *__restrict__ tab, long long plane,
-                                        long long off, Geo &g) {
+__device__ __forceinline__ int load_geo(const double *__restrict__ tab, Geo &g) {
   constexpr TabLayout L = tab_layout(MT);
   double cov[L.nsym], con[L.ncon];
 #pragma unroll
-  for (int q = 0; q < L.nsym; ++q) cov[q] = __ldg(tab + off + q * plane);
+  for (int q = 0; q < L.nsym; ++q) cov[q] = __ldg(tab + q * kTabCols);
 #pragma unroll
-  for (int q = 0; q < L.ncon; ++q) con[q] = __ldg(tab + off + (L.nsym + q) * plane);
+  for (int q = 0; q < L.ncon; ++q) con[q] = __ldg(tab + (L.nsym + q) * kTabCols);
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -271,24 +287,23 @@ __device__ __forceinline__ int load_geo(const double *__restrict__ tab, long lon
       g.gcov[r][c] = L.sym[r][c] >= 0 ? cov[L.sym[r][c]] : 0.0;
       g.gcon[r][c] = L.con[r][c] >= 0 ? con[L.con[r][c]] : 0.0;
     }
-  const long long s0 = L.nsym + L.ncon;
-  g.gdet = __ldg(tab + off + s0 * plane);
-  g.sg = __ldg(tab + off + (s0 + 1) * plane);
-  g.alpha = __ldg(tab + off + (s0 + 2) * plane);
-  return __ldg(tab + off + (s0 + 3) * plane) != 0.0;
+  constexpr int s0 = L.nsym + L.ncon;
+  g.gdet = __ldg(tab + s0 * kTabCols);
+  g.sg = __ldg(tab + (s0 + 1) * kTabCols);
+  g.alpha = __ldg(tab + (s0 + 2) * kTabCols);
+  return __ldg(tab + (s0 + 3) * kTabCols) != 0.0;
 }
 
 #if PGK_MIXED
 // load_geo from an FP32 copy of a table: the values geo_cast would give.
 template <int MT>
-__device__ __forceinline__ int load_geo_f32(const float *__restrict__ tab, long long plane,
-                                            long long off, GeoT<float> &g) {
+__device__ __forceinline__ int load_geo_f32(const float *__restrict__ tab, GeoT<float> &g) {
   constexpr TabLayout L = tab_layout(MT);
   float cov[L.nsym], con[L.ncon];
 #pragma unroll
-  for (int q = 0; q < L.nsym; ++q) cov[q] = __ldg(tab + off + q * plane);
+  for (int q = 0; q < L.nsym; ++q) cov[q] = __ldg(tab + q * kTabCols);
 #pragma unroll
-  for (int q = 0; q < L.ncon; ++q) con[q] = __ldg(tab + off + (L.nsym + q) * plane);
+  for (int q = 0; q < L.ncon; ++q) con[q] = __ldg(tab + (L.nsym + q) * kTabCols);
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -296,11 +311,11 @@ __device__ __forceinline__ int load_geo_f32(const float *__restrict__ tab, long 
       g.gcov[r][c] = L.sym[r][c] >= 0 ? cov[L.sym[r][c]] : 0.0f;
       g.gcon[r][c] = L.con[r][c] >= 0 ? con[L.con[r][c]] : 0.0f;
     }
-  const long long s0 = L.nsym + L.ncon;
-  g.gdet = __ldg(tab + off + s0 * plane);
-  g.sg = __ldg(tab + off + (s0 + 1) * plane);
-  g.alpha = __ldg(tab + off + (s0 + 2) * plane);
-  return __ldg(tab + off + (s0 + 3) * plane) != 0.0f;
+  constexpr int s0 = L.nsym + L.ncon;
+  g.gdet = __ldg(tab + s0 * kTabCols);
+  g.sg = __ldg(tab + (s0 + 1) * kTabCols);
+  g.alpha = __ldg(tab + (s0 + 2) * kTabCols);
+  return __ldg(tab + (s0 + 3) * kTabCols) != 0.0f;
 }
 #endif
 
@@ -331,8 +346,7 @@ __device__ __forceinline__ int cell_metric(const Dims &d, const pangu_params &p,
                                            int j, int i, Geo &g) {
   if (MT == MKS || MT == BL) {
     constexpr TabLayout L = tab_layout(MT);
-    const long long plane = (long long)d.N2 * d.N1;
-    return load_geo<MT>(d.ctab, plane, (long long)b * L.ncen * plane + (long long)j * d.N1 + i, g);
+    return load_geo<MT>(d.ctab + tab_at(L.ncen, d.N2, d.N1, b, j, i), g);
   } else if (MT == CKS) {
     const double x[4] = {0.0, xc(d, b, 0, i), xc(d, b, 1, j), xc(d, b, 2, k)};
     return analytic_geo<MT>(d, p, b, i, 0, j, 0, x, g);
@@ -342,21 +356,33 @@ __device__ __forceinline__ int cell_metric(const Dims &d, const pangu_params &p,
   }
 }
 
+#if PGK_MIXED
+// cell_metric rounded to FP32: from the FP32 copy of the centre table (half the
+// bytes and no conversions), or cast.
+template <int MT>
+__device__ __forceinline__ int cell_metric_f32(const Dims &d, const pangu_params &p, int b, int k,
+                                               int j, int i, GeoT<FT> &g) {
+  if (MT == MKS || MT == BL) {
+    constexpr TabLayout L = tab_layout(MT);
+    return load_geo_f32<MT>(d.ctab32 + tab_at(L.ncen, d.N2, d.N1, b, j, i), g);
+  }
+  Geo g64;
+  const int ok = cell_metric<MT>(d, p, b, k, j, i, g64);
+  geo_cast<MT>(g64, g);
+  return ok;
+}
+#endif
+
 // Metric at the lower face of (b, k, j, i) along dir (1..3).
 template <int MT>
 __device__ __forceinline__ int face_metric(const Dims &d, const pangu_params &p, int dir, int b,
                                            int k, int j, int i, Geo &g) {
   if (MT == MKS || MT == BL) {
     constexpr TabLayout L = tab_layout(MT);
-    if (dir == 1) {
-      const long long plane = (long long)d.N2 * (d.N1 + 1);
-      return load_geo<MT>(d.f1tab, plane,
-                          (long long)b * L.nmet * plane + (long long)j * (d.N1 + 1) + i, g);
-    } else if (dir == 2) {
-      const long long plane = (long long)(d.N2 + 1) * d.N1;
-      return load_geo<MT>(d.f2tab, plane, (long long)b * L.nmet * plane + (long long)j * d.N1 + i,
-                          g);
-    }
+    if (dir == 1)
+      return load_geo<MT>(d.f1tab + tab_at(L.nmet, d.N2, d.N1 + 1, b, j, i), g);
+    else if (dir == 2)
+      return load_geo<MT>(d.f2tab + tab_at(L.nmet, d.N2 + 1, d.N1, b, j, i), g);
     return cell_metric<MT>(d, p, b, k, j, i, g);  // independent of x3
   } else if (MT == CKS) {
     const double x[4] = {0.0, dir == 1 ? xf(d, b, 0, i) : xc(d, b, 0, i),
@@ -455,7 +481,7 @@ template <int MT>
 // (with_b = 0: conserved B left as is, see k_calc_cons).
 // zero0, zero1 (may be null) are list counters of later tasks of the stage,
 // set to 0 here so that the stage needs no memset.
-__global__ void __launch_bounds__(kThreads, 4) k_fix_primitive(Dims d, pangu_params p, PT *P,
+__global__ void __launch_bounds__(kFixThreads, 6) k_fix_primitive(Dims d, pangu_params p, PT *P,
                                                             unsigned long long *cnt, double *U,
                                                             int with_cons, int with_b, int *zero0,
                                                             int *zero1) {
@@ -594,18 +620,48 @@ __global__ void __launch_bounds__(kThreads, 4) k_fix_primitive(Dims d, pangu_par
     u2 *= f;
     u3 *= f;
   }
+  const bool excised = MT == CKS && r < p.r_excise;
   const double rho_after = kmax(pr, small);
-  double kel = pc[KEL];
-  if (p.enable_heating && rho_after != rho_before) kel *= PGK_POW(rho_after / rho_before, -gam);
-  double ent = (gam - 1.0) * pu * PGK_POW(pr, -gam);
-  if (p.enable_heating) kel = clamp_by_ratio(p.ratio_min, p.ratio_max, ent, kel);
-  if (MT == CKS && r < p.r_excise) {
-    const double e_excise = p.pexcise / (gam - 1.0);
+  const double e_excise = p.pexcise / (gam - 1.0);
+  if (excised) {
     pr = p.dexcise;
     pu = e_excise;
     u1 = u2 = u3 = 0.0;
+  }
+  // The conserved variables but the entropies', before the powers below: the
+  // state then need not stay in registers across them. It depends on the
+  // velocity and the field only, so it is the one above unless the velocity was
+  // changed.
+  const bool cons = with_cons && k >= d.ks && k <= d.ke && j >= d.js && j <= d.je && i >= d.is &&
+                    i <= d.ie;
+  double f_rho = 0.0;
+  if (cons) {
+    pc[RHO] = pr;
+    pc[ENY] = pu;
+    pc[UX1] = u1;
+    pc[UX2] = u2;
+    pc[UX3] = u3;
+    if (cap || excised) calc_state<MT>(pc, g, st);
+    double f[NPRIM];
+    flux_from_state(gam, pc, st, g.sg, 0, f);
+#pragma unroll
+    for (int v = 0; v < ENT; ++v)
+      if (d.pidx[v] >= 0 && (with_b || v < BX1)) a_cons(d, U, b, d.pidx[v])[o] = f[v];
+    f_rho = pr * st.ucon[0];
+  }
+  double kel = pc[KEL];
+  double ent;
+  if (excised) {
     ent = (gam - 1.0) * e_excise * PGK_POW(p.dexcise, -gam);
-    if (p.enable_heating) kel = e_excise;
+    kel = e_excise;
+  } else {
+    if (p.enable_heating && rho_after != rho_before) kel *= PGK_POW(rho_after / rho_before, -gam);
+    ent = (gam - 1.0) * pu * PGK_POW(pr, -gam);
+    if (p.enable_heating) kel = clamp_by_ratio(p.ratio_min, p.ratio_max, ent, kel);
+  }
+  if (cons) {
+    a_cons(d, U, b, d.pidx[ENT])[o] = ent * f_rho * g.sg;
+    if (d.pidx[KEL] >= 0) a_cons(d, U, b, d.pidx[KEL])[o] = kel * f_rho * g.sg;
   }
 #endif
   a_prim(d, P, b, 0)[o] = pr;
@@ -618,6 +674,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_fix_primitive(Dims d, pangu_par
   count(cnt, job_of(d, b), PANGU_CNT_RHO_FLOOR, hit_r);
   count(cnt, job_of(d, b), PANGU_CNT_ENG_FLOOR, hit_u);
   count(cnt, job_of(d, b), PANGU_CNT_LORENTZ_CAP, cap);
+#if PGK_MIXED
   if (with_cons && k >= d.ks && k <= d.ke && j >= d.js && j <= d.je && i >= d.is && i <= d.ie) {
     // the stored values, as a reload would see them
     double pf[NPRIM];
@@ -630,14 +687,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_fix_primitive(Dims d, pangu_par
     pf[UX3] = (PT)u3;
     pf[ENT] = (PT)ent;
     if (p.enable_heating) pf[KEL] = (PT)kel;
-    State sf;
-    calc_state<MT>(pf, g, sf);
+    State st;
+    calc_state<MT>(pf, g, st);
     double f[NPRIM];
-    flux_from_state(gam, pf, sf, g.sg, 0, f);
+    flux_from_state(gam, pf, st, g.sg, 0, f);
 #pragma unroll
     for (int v = 0; v < NPRIM; ++v)
       if (d.pidx[v] >= 0 && (with_b || v < BX1 || v > BX3)) a_cons(d, U, b, d.pidx[v])[o] = f[v];
   }
+#endif
 }
 
 // ---------------------------------------------------------------------------
@@ -706,6 +764,8 @@ template <int MT, int DIR>
 __device__ __forceinline__ void face_geo(const Dims &d, const pangu_params &p, int b, int k, int j,
                                          int i, FaceGeo &fg) {
 #if !PGK_MIXED
+  // not hoisted above the reconstruction, where its registers spill
+  asm volatile("" : "+r"(i));
   fg.ok = face_metric<MT>(d, p, DIR, b, k, j, i, fg.g);
 #endif
 }
@@ -932,15 +992,10 @@ __device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, 
   if ((MT == MKS || MT == BL) && DIR != 3) {
     // the FP32 face tables (pool_init builds them for every mixed engine)
     constexpr TabLayout L = tab_layout(MT);
-    if (DIR == 1) {
-      const long long plane = (long long)d.N2 * (d.N1 + 1);
-      ok = load_geo_f32<MT>(d.f1tab32, plane,
-                            (long long)b * L.nmet * plane + (long long)j * (d.N1 + 1) + i, g);
-    } else {
-      const long long plane = (long long)(d.N2 + 1) * d.N1;
-      ok = load_geo_f32<MT>(d.f2tab32, plane, (long long)b * L.nmet * plane + (long long)j * d.N1 + i,
-                            g);
-    }
+    ok = DIR == 1 ? load_geo_f32<MT>(d.f1tab32 + tab_at(L.nmet, d.N2, d.N1 + 1, b, j, i), g)
+                  : load_geo_f32<MT>(d.f2tab32 + tab_at(L.nmet, d.N2 + 1, d.N1, b, j, i), g);
+  } else if (MT == MKS || MT == BL) {
+    ok = cell_metric_f32<MT>(d, p, b, k, j, i, g);  // independent of x3
   } else {
     Geo g64;
     ok = face_metric<MT>(d, p, DIR, b, k, j, i, g64);
@@ -1097,10 +1152,10 @@ __device__ __forceinline__ void face_flux_split(const Dims &d, const pangu_param
   }
   const double gam = p.adiabatic_index;
   const double sg = g.sg;
-  const xd::Rcp al = xd::rcp(g.alpha);
   const bool al_ok = xd::in_range_den(g.alpha);
   double vmaxL, vminL;
   {
+    const xd::Rcp al = xd::rcp(g.alpha);
     double P[NPRIM];
 #pragma unroll
     for (int s = 0; s < NPRIM; ++s) P[s] = sl[s * ss];
@@ -1121,6 +1176,11 @@ __device__ __forceinline__ void face_flux_split(const Dims &d, const pangu_param
   for (int s = 0; s < NPRIM; ++s) P[s] = sr[s * ss];
   State st;
   double vmaxR, vminR;
+  // formed again rather than kept over the left side (six registers); the
+  // assembly keeps the compiler from seeing that it is the same
+  double lapse = g.alpha;
+  asm volatile("" : "+d"(lapse));
+  const xd::Rcp al = xd::rcp(lapse);
   face_side<MT, DIR>(gam, P, g, al, al_ok, st, vmaxR, vminR);
   const FluxOf<DIR> f(gam, P, st);
   const FluxOf<0> u(gam, P, st);
@@ -1150,13 +1210,20 @@ constexpr int kFacesPerWarp = 31;
 // three; 3 CTAs with 168 registers: 56 us and 3.17 ms).
 constexpr int kFluxThreads = 128;
 constexpr int kFluxBlocks = 4;
+// The mixed form's tabulated-metric kernels need 72 registers with one face's
+// reconstruction in flight and 96 with a march; bounds that say so keep ptxas
+// from taking 80 and 108 (x1 947 against 1052 us per cycle on the 3D torus, x2
+// and x3 1576 against 1758).
+constexpr int flux_blocks(int mt, bool march) {
+  return !PGK_MIXED || mt == CKS ? kFluxBlocks : (march ? 5 : 7);
+}
 // FP64, curved metrics: one side's state in registers at a time
 // (face_flux_split; 47 against 49 us on the 2D torus, 2.41 against 2.52 ms on
 // the 3D one). Minkowski keeps both (its metric takes no registers).
 constexpr bool split_faces(int mt) { return PGK_SPLIT_FACES && mt != MINKOWSKI; }
 
 template <int MT, int OPT>
-__global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_x1(Dims d, pangu_params p, int k0, int k1,
+__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT, false)) k_flux_x1(Dims d, pangu_params p, int k0, int k1,
                                                       int j0, int j1, int i0, int i1,
                                                       const PT *P, double *F,
                                                       double *alfven) {
@@ -1211,6 +1278,56 @@ __global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_x1(Dims d, p
   for (int s = 0; s < NPRIM; ++s) PL[s] = __shfl_up_sync(0xffffffffu, PL[s], 1);
   if (lane == 0 || !active) return;
   FaceGeo fg;
+  face_geo<MT, 1>(d, p, b, k, j, c, fg);
+  face_flux<MT, 1, OPT>(d, p, fg, b, k, j, c, PL, PR, F, alfven);
+}
+
+// The last faces f0 .. f1 of every row, fewer than a warp's share: a row takes
+// G lanes (a power of two above the number of faces), so a warp takes 32 / G
+// rows. Lane l of a row's group holds cell f0 - 1 + l, as in k_flux_x1.
+template <int MT, int OPT>
+__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT, false))
+    k_flux_x1_rest(Dims d, pangu_params p, int k0, int k1, int j0, int j1, int f0, int f1, int G,
+                   const PT *P, double *F, double *alfven) {
+  pdl_grid_wait();
+  const int lane = threadIdx.x & 31, l = lane & (G - 1);
+  const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const long long nrow = (long long)(k1 - k0 + 1) * (j1 - j0 + 1);
+  const long long last = nrow * d.NB - 1;
+  long long rr, jr;
+  const int bb = (int)div_fast(min(row, last), nrow, rr);
+  const int b = slot_of(d, bb);
+  const int k = k0 + (int)div_fast(rr, j1 - j0 + 1, jr);
+  const int j = j0 + (int)jr;
+  const int c = f0 - 1 + l;
+  const bool active = row <= last && c <= f1;
+  // an inactive lane reads the last cell's stencil
+  auto cell = [&](int v) { return a_prim(d, P, b, v) + coff(d, k, j, min(c, f1)); };
+  FaceGeo fg;
+#if PGK_SPLIT_FACES
+  if (split_faces(MT)) {
+    extern __shared__ double fsm[];  // as in k_flux_x1
+    const int ss = blockDim.x, t = threadIdx.x;
+    recon_vars<OPT>(d, p, cell, 1, [&](int s, FT up, FT lo) {
+      fsm[s * ss + t] = up;
+      fsm[(NPRIM + s) * ss + t] = lo;
+    });
+    __syncwarp();
+    if (l == 0 || !active) return;
+    face_geo<MT, 1>(d, p, b, k, j, c, fg);
+    face_flux_split<MT, 1, OPT>(d, p, fg, b, k, j, c, fsm + t - 1, fsm + NPRIM * ss + t,
+                                fsm + 2 * NPRIM * ss + t, ss, F, alfven);
+    return;
+  }
+#endif
+  FT PL[NPRIM], PR[NPRIM];
+  recon_vars<OPT>(d, p, cell, 1, [&](int s, FT up, FT lo) {
+    PL[s] = up;
+    PR[s] = lo;
+  });
+#pragma unroll
+  for (int s = 0; s < NPRIM; ++s) PL[s] = __shfl_up_sync(0xffffffffu, PL[s], 1);
+  if (l == 0 || !active) return;
   face_geo<MT, 1>(d, p, b, k, j, c, fg);
   face_flux<MT, 1, OPT>(d, p, fg, b, k, j, c, PL, PR, F, alfven);
 }
@@ -1664,7 +1781,7 @@ __global__ void __launch_bounds__(32 * kTmaRowsX1, kFluxBlocks)
 }
 
 template <int MT, int MARCH, int OPT>
-__global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_march2(Dims d, pangu_params p, int k0, int k1,
+__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT, MARCH > 1)) k_flux_march2(Dims d, pangu_params p, int k0, int k1,
                                                           int j0, int j1, int i0, int i1,
                                                           const PT *P, double *F,
                                                           double *alfven) {
@@ -1672,7 +1789,7 @@ __global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_march2(Dims 
   flux_march_body<MT, 2, MARCH, OPT>(d, p, k0, k1, j0, j1, i0, i1, P, F, alfven);
 }
 template <int MT, int MARCH, int OPT>
-__global__ void __launch_bounds__(kFluxThreads, kFluxBlocks) k_flux_march3(Dims d, pangu_params p, int k0, int k1,
+__global__ void __launch_bounds__(kFluxThreads, flux_blocks(MT, MARCH > 1)) k_flux_march3(Dims d, pangu_params p, int k0, int k1,
                                                           int j0, int j1, int i0, int i1,
                                                           const PT *P, double *F,
                                                           double *alfven) {
@@ -1953,16 +2070,15 @@ __device__ __forceinline__ void source_cell(const Dims &d, const pangu_params &p
 #pragma unroll
     for (int v = 0; v < NPRIM; ++v) pf[v] = d.pidx[v] >= 0 ? a_prim(d, P, b, d.pidx[v])[q0] : FT(0);
     GeoT<FT> gf;
-    geo_cast<MT>(g, gf);
+    cell_metric_f32<MT>(d, p, b, k, j, i, gf);
     StateT<FT> sf;
     calc_state_t<MT>(pf, gf, sf);
     const FT gam = (FT)p.adiabatic_index;
     const FT hh = pf[RHO] + gam * pf[ENY];
     const FT e_tot = hh + sf.bsq;
     const FT p_tot = (gam - FT(1)) * pf[ENY] + FT(0.5) * sf.bsq;
-    const long long plane = (long long)d.N2 * d.N1;
-    // the FP32 Christoffel planes (pool_init builds them for every mixed engine)
-    const float *cn = d.ctab32 + (long long)b * L.nconn * plane + (long long)j * d.N1 + i;
+    // the FP32 Christoffel symbols (pool_init builds them for every mixed engine)
+    const float *cn = d.ctab32 + tab_at(L.ncen, d.N2, d.N1, b, j, i) + L.nmet * kTabCols;
 #pragma unroll
     for (int dir = 0; dir < 4; ++dir) {
       FT con = FT(0);
@@ -1973,7 +2089,7 @@ __device__ __forceinline__ void source_cell(const Dims &d, const pangu_params &p
           if (L.conn[c][dir][r] >= 0) {
             const FT T = e_tot * sf.ucon[r] * sf.ucov[c] + p_tot * FT(r == c) -
                          sf.bcon[r] * sf.bcov[c];
-            con += T * (FT)__ldg(cn + L.conn[c][dir][r] * plane);
+            con += T * (FT)__ldg(cn + L.conn[c][dir][r] * kTabCols);
           }
       const int v = dir == 0 ? d.pidx[ENY] : d.pidx[UX1] + dir - 1;
       a_cons(d, U, b, v)[q0] += (double)con * sg * bdt;
@@ -1991,9 +2107,7 @@ __device__ __forceinline__ void source_cell(const Dims &d, const pangu_params &p
   if (MT == MKS || MT == BL) {
     // Christoffel symbols from the centre table; structural zeros skipped
     constexpr TabLayout L = tab_layout(MT);
-    const long long plane = (long long)d.N2 * d.N1;
-    const double *cn = d.ctab + (long long)b * L.ncen * plane + (long long)j * d.N1 + i +
-                       (long long)L.nmet * plane;
+    const double *cn = d.ctab + tab_at(L.ncen, d.N2, d.N1, b, j, i) + L.nmet * kTabCols;
     // the four contractions first, then the four updates: no Christoffel load
     // waits behind a store to U
     double con[4];
@@ -2005,7 +2119,7 @@ __device__ __forceinline__ void source_cell(const Dims &d, const pangu_params &p
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (L.conn[c][dir][r] >= 0)
-            con[dir] += T[r][c] * __ldg(cn + L.conn[c][dir][r] * plane);
+            con[dir] += T[r][c] * __ldg(cn + L.conn[c][dir][r] * kTabCols);
     }
     const long long q = coff(d, k, j, i);
     double u[4];
@@ -2043,7 +2157,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_source(Dims d, pangu_params p, 
   b = slot_of(d, b);
   if (MT == MINKOWSKI) return;
   Geo g;
-  cell_metric<MT>(d, p, b, k, j, i, g);
+#if PGK_MIXED
+  if (MT == MKS || MT == BL) {  // the FP32 source term reads its own copy
+    constexpr TabLayout L = tab_layout(MT);
+    g.sg = __ldg(d.ctab + tab_at(L.ncen, d.N2, d.N1, b, j, i) + (L.nsym + L.ncon + 1) * kTabCols);
+  } else
+#endif
+    cell_metric<MT>(d, p, b, k, j, i, g);
   source_cell<MT>(d, p, P, U, b, k, j, i, g, beta * dt[job_of(d, b)]);
 }
 
@@ -2062,24 +2182,24 @@ __global__ void __launch_bounds__(kThreads) k_build_tables(Dims d, pangu_params 
   const int bb = (int)(t / per);
   t -= (long long)bb * per;
   const int b = slot_of(d, bb);
-  int which, W;
-  long long plane;
+  int which, W, R = d.N2;
+  constexpr int plane = kTabCols;
   double *tab;
   int nc;
   if (t < pc) {
-    which = 0, W = d.N1, plane = pc, tab = ctab, nc = L.ncen;
+    which = 0, W = d.N1, tab = ctab, nc = L.ncen;
   } else if (t < pc + p1) {
     t -= pc;
-    which = 1, W = d.N1 + 1, plane = p1, tab = f1tab, nc = L.nmet;
+    which = 1, W = d.N1 + 1, tab = f1tab, nc = L.nmet;
   } else {
     t -= pc + p1;
-    which = 2, W = d.N1, plane = p2, tab = f2tab, nc = L.nmet;
+    which = 2, W = d.N1, R = d.N2 + 1, tab = f2tab, nc = L.nmet;
   }
   const int j = (int)(t / W), i = (int)(t % W);
   const double x[4] = {0.0, 0.0, 0.0, 0.0};
   Geo g;
   const int ok = analytic_geo<MT>(d, p, b, i, which == 1 ? 3 : 0, j, which == 2 ? 3 : 0, x, g);
-  double *o = tab + (long long)b * nc * plane + t;
+  double *o = tab + tab_at(nc, R, W, b, j, i);
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -2087,7 +2207,7 @@ __global__ void __launch_bounds__(kThreads) k_build_tables(Dims d, pangu_params 
       if (c >= r && L.sym[r][c] >= 0) o[L.sym[r][c] * plane] = g.gcov[r][c];
       if (L.con[r][c] >= 0) o[(L.nsym + L.con[r][c]) * plane] = g.gcon[r][c];
     }
-  const long long s0 = L.nsym + L.ncon;
+  constexpr int s0 = L.nsym + L.ncon;
   o[s0 * plane] = g.gdet;
   o[(s0 + 1) * plane] = g.sg;
   o[(s0 + 2) * plane] = g.alpha;
@@ -2105,36 +2225,16 @@ __global__ void __launch_bounds__(kThreads) k_build_tables(Dims d, pangu_params 
   }
 }
 
-// Mixed form: ncomp planes of a slot-major table, for the job's slots,
-// rounded once to FP32.
-__global__ void __launch_bounds__(kThreads) k_planes_to_f32(Dims d, const double *src, float *dst,
-                                                            int ncomp, long long plane) {
+// Mixed form: a table of the job's slots (n entries each) rounded once to FP32.
+__global__ void __launch_bounds__(kThreads) k_table_to_f32(Dims d, const double *src, float *dst,
+                                                           long long n) {
   pdl_grid_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)d.NB * ncomp * plane) return;
-  long long off, q;
-  const long long bq = div_fast(t, plane, off);
-  const int bb = (int)div_fast(bq, ncomp, q);
-  const long long at = ((long long)slot_of(d, bb) * ncomp + q) * plane + off;
+  if (t >= (long long)d.NB * n) return;
+  long long off;
+  const int bb = (int)div_fast(t, n, off);
+  const long long at = (long long)slot_of(d, bb) * n + off;
   dst[at] = (float)src[at];
-}
-
-// Mixed form: the centre table's Christoffel planes of the job's slots
-// rounded once to FP32 (what the FP32 source term converts each value to
-// anyway), so that the source term reads half the bytes.
-template <int MT>
-__global__ void __launch_bounds__(kThreads) k_conn_to_f32(Dims d, float *out) {
-  pdl_grid_wait();
-  constexpr TabLayout L = tab_layout(MT);
-  const long long plane = (long long)d.N2 * d.N1;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)d.NB * L.nconn * plane) return;
-  long long off, q;
-  const long long bq = div_fast(t, plane, off);
-  const int bb = (int)div_fast(bq, L.nconn, q);
-  const long long sl = slot_of(d, bb);
-  out[(sl * L.nconn + q) * plane + off] =
-      (float)d.ctab[(sl * L.ncen + L.nmet + q) * plane + off];
 }
 
 // ---------------------------------------------------------------------------
@@ -2142,38 +2242,10 @@ __global__ void __launch_bounds__(kThreads) k_conn_to_f32(Dims d, float *out) {
 // ---------------------------------------------------------------------------
 // Electron heating of one interior cell from its primitives and conserved
 // variables as they stand in memory: writes the electron entropy. The mixed
-// form computes the state and the heating in FT (FP32).
-template <int MT>
-__device__ __forceinline__ void heat_cell(const Dims &d, const pangu_params &p, PT *P,
-                                          const double *U, int b, int k, int j, int i,
-                                          const Geo &g) {
-  const long long q = coff(d, k, j, i);
-  const double cr = a_cons(d, U, b, 0)[q];
-  const HeatParams hp = {p.model, p.adiabatic_index, p.gamma_p, p.gamma_e, p.fel_constant,
-                         p.ratio_min, p.ratio_max, p.limit_kel, p.suppress_highb_heat,
-                         p.enforce_positive_dissipation};
-#if PGK_MIXED
-  FT pc[NPRIM];
-#pragma unroll
-  for (int v = 0; v < NPRIM; ++v) pc[v] = d.pidx[v] >= 0 ? a_prim(d, P, b, d.pidx[v])[q] : FT(0);
-  GeoT<FT> gf;
-  geo_cast<MT>(g, gf);
-  StateT<FT> s;
-  calc_state_t<MT>(pc, gf, s);
-  a_prim(d, P, b, d.pidx[KEL])[q] =
-      heating_apply_t<FT>(hp, pc[RHO], pc[ENY], s.bsq, (FT)(a_cons(d, U, b, d.pidx[ENT])[q] / cr),
-                          pc[ENT], (FT)(a_cons(d, U, b, d.pidx[KEL])[q] / cr));
-#else
-  double pc[NPRIM];
-  load_prim(d, P, b, k, j, i, pc);
-  State s;
-  calc_state<MT>(pc, g, s);
-  a_prim(d, P, b, d.pidx[KEL])[q] =
-      heating_apply(hp, pc[RHO], pc[ENY], s.bsq, a_cons(d, U, b, d.pidx[ENT])[q] / cr, pc[ENT],
-                    a_cons(d, U, b, d.pidx[KEL])[q] / cr);
-#endif
-}
-
+// form computes the state and the heating in FT (FP32). Only the models that
+// read b^2 (and the suppression at high magnetisation) need the metric and the
+// state: the constant and the Sharma model skip both (187 to 104 us per stage on
+// the 3D torus, 10 to 7.4 on the 2D one).
 template <int MT>
 __global__ void __launch_bounds__(kThreads, 4) k_heating(Dims d, pangu_params p, PT *P,
                                                       const double *U) {
@@ -2182,9 +2254,47 @@ __global__ void __launch_bounds__(kThreads, 4) k_heating(Dims d, pangu_params p,
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (!box_index(t, d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie, b, k, j, i)) return;
   b = slot_of(d, b);
-  Geo g;
-  cell_metric<MT>(d, p, b, k, j, i, g);
-  heat_cell<MT>(d, p, P, U, b, k, j, i, g);
+  const long long q = coff(d, k, j, i);
+  const double cr = a_cons(d, U, b, 0)[q];
+  const double ce = a_cons(d, U, b, d.pidx[ENT])[q], ck = a_cons(d, U, b, d.pidx[KEL])[q];
+  const FT rho = a_prim(d, P, b, 0)[q], eny = a_prim(d, P, b, 1)[q],
+           ent = a_prim(d, P, b, d.pidx[ENT])[q];
+  const HeatParams hp = {p.model, p.adiabatic_index, p.gamma_p, p.gamma_e, p.fel_constant,
+                         p.ratio_min, p.ratio_max, p.limit_kel, p.suppress_highb_heat,
+                         p.enforce_positive_dissipation};
+  FT bsq = 0;
+  if (p.suppress_highb_heat || (p.model != 0 && p.model != 5)) {
+#if PGK_MIXED
+    FT pc[NPRIM];
+#pragma unroll
+    for (int v = 0; v < NPRIM; ++v) pc[v] = d.pidx[v] >= 0 ? a_prim(d, P, b, d.pidx[v])[q] : FT(0);
+    GeoT<FT> gf;
+    cell_metric_f32<MT>(d, p, b, k, j, i, gf);
+    StateT<FT> s;
+    calc_state_t<MT>(pc, gf, s);
+    bsq = s.bsq;
+#else
+    Geo g;
+    cell_metric<MT>(d, p, b, k, j, i, g);
+    double pc[NPRIM];
+    load_prim(d, P, b, k, j, i, pc);
+    State s;
+    calc_state<MT>(pc, g, s);
+    bsq = s.bsq;
+#endif
+  }
+#if PGK_MIXED
+  a_prim(d, P, b, d.pidx[KEL])[q] =
+      heating_apply_t<FT>(hp, rho, eny, bsq, (FT)(ce / cr), ent, (FT)(ck / cr));
+#else
+  const xd::Rcp ic = xd::rcp(cr);
+  double tot = xd::quot_s(ce, ic), el = xd::quot_s(ck, ic);
+  if (!(xd::in_range_den(cr) & (cr > 0.0) & xd::in_range0(ce) & xd::in_range0(ck))) {
+    tot = div_plain(ce, cr);
+    el = div_plain(ck, cr);
+  }
+  a_prim(d, P, b, d.pidx[KEL])[q] = heating_apply(hp, rho, eny, bsq, tot, ent, el);
+#endif
 }
 
 // ---------------------------------------------------------------------------
@@ -2333,7 +2443,7 @@ __global__ void __launch_bounds__(kRecoveryThreads, 7) k_recovery(Dims d, pangu_
 }
 
 template <int MT>
-__global__ void __launch_bounds__(kRecoveryThreads, 7)
+__global__ void __launch_bounds__(kRecoveryThreads, 6)
     k_recovery_chain(Dims d, pangu_params p, PT *P, const double *U, double *flag,
                      unsigned long long *cnt, int *nfix, long long *fix) {
   pdl_grid_wait();
@@ -2985,7 +3095,8 @@ int run_fix_primitive(pangu_engine *e, const pangu_pack *md, bool with_cons, cud
   const long long n = (long long)d.NB * d.ncell;
   // on the stage path (with_cons) the C2P retry and FixRecovery list counters
   // are zeroed here for Recovery
-  DISPATCH_MT(e->p.metric_type, k_fix_primitive, grid_for(n), s, d, e->p, prim_of(md), e->d_cnt,
+  DISPATCH_MT_T(e->p.metric_type, k_fix_primitive, (unsigned)((n + kFixThreads - 1) / kFixThreads), kFixThreads,
+                s, d, e->p, prim_of(md), e->d_cnt,
               md->cons, with_cons ? 1 : 0, PGK_MIXED ? 0 : 1,
               with_cons ? e->d_fail_count : nullptr, with_cons ? e->d_fix_count : nullptr);
   ++e->launches;
@@ -3054,6 +3165,23 @@ inline bool tma_tile_map(const pangu_engine *e, const pangu_pack *md, int dir, C
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Lanes per row of k_flux_x1_rest, or 0 where the x1 kernel takes every face: a
+// row of nf faces fills nf / 31 warps and leaves nf % 31 faces, which as a
+// segment of their own cost a whole warp. Packed, they cost G / 32 of one and a
+// launch; worth it where the warps saved fill the GPU once (16 per SM, about
+// 15 us of x1 work, against 2 to 4 us for a launch). 64^3 blocks have 65 faces:
+// 2.1 warps a row for 3 (x1 XXX against YYY us per cycle on the 3D torus), 32^3
+// blocks 33: 1.1 for 2.
+inline int x1_rest_lanes(const Dims &d) {
+  const int nf = d.ie + 1 - d.is + 1, rest = nf % kFacesPerWarp;
+  if (rest == 0 || nf < kFacesPerWarp) return 0;
+  int G = 2;
+  while (G < rest + 1) G *= 2;
+  if (G > 16) return 0;
+  const long long rows = (long long)d.NB * (d.ke - d.ks + 1 + 2 * d.o3) * (d.je - d.js + 1 + 2 * d.o2);
+  return rows * (32 - G) / 32 >= 16LL * device_sms() ? G : 0;
+}
+
 // Launches the flux kernel of one direction with a given march depth
 // (x2/x3) and CTA size. The TMA-staged kernels read the contiguous layout; a
 // pack whose primitives come through a table runs the thread-loaded form of
@@ -3068,6 +3196,7 @@ void launch_flux_dir(const pangu_engine *e, const pangu_pack *md, int dir, int m
   int k0 = d.ks - d.o3, k1 = d.ke + d.o3, j0 = d.js - d.o2, j1 = d.je + d.o2;
   int i0 = d.is - d.o1, i1 = d.ie + d.o1;
   if (dir == 1) { i0 = d.is; i1 = d.ie + 1; }
+  const int rest = dir == 1 ? x1_rest_lanes(d) : 0;
   if (dir == 2) { j0 = d.js; j1 = d.je + 1; }
   if (dir == 3) {  // hll.cc:293-296 narrows the transverse range
     k0 = d.ks; k1 = d.ke + 1;
@@ -3075,9 +3204,19 @@ void launch_flux_dir(const pangu_engine *e, const pangu_pack *md, int dir, int m
   }
   double *F = dir == 1 ? md->flux1 : (dir == 2 ? md->flux2 : md->flux3);
   const PT *P = prim_of(md);
+  CUtensorMap tm;
+  if (dir == 1 && march == kMarchTma && !tma_tile_map(e, md, 1, &tm))
+    return;  // pangu_set_flux_config checked tma_ok
+  if (rest) {
+    const int f0 = i1 - (i1 - i0 + 1) % kFacesPerWarp + 1;
+    const long long rows = (long long)d.NB * (k1 - k0 + 1) * (j1 - j0 + 1);
+    launch_pdl_smem(k_flux_x1_rest<MT, OPT>, dim3(grid_flux(rows * rest, kFluxThreads)),
+                    dim3(kFluxThreads),
+                    split_faces(MT) ? 3 * NPRIM * kFluxThreads * sizeof(double) : 0, s, d, e->p,
+                    k0, k1, j0, j1, f0, i1, rest, P, F, md->alfven);
+    i1 = f0 - 1;
+  }
   if (dir == 1 && march == kMarchTma) {
-    CUtensorMap tm;
-    if (!tma_tile_map(e, md, 1, &tm)) return;  // pangu_set_flux_config checked tma_ok
     const int nseg = (i1 - i0 + 1 + kFacesPerWarp - 1) / kFacesPerWarp;
     const long long nt = (long long)d.NB * (k1 - k0 + 1) *
                          ((j1 - j0 + 1 + kTmaRowsX1 - 1) / kTmaRowsX1) * nseg;
@@ -3097,7 +3236,6 @@ void launch_flux_dir(const pangu_engine *e, const pangu_pack *md, int dir, int m
   const int m = dir == 2 ? (j1 - j0 + 1) : (k1 - k0 + 1);
   const int na = dir == 2 ? (k1 - k0 + 1) : (j1 - j0 + 1);
   if (march == kMarchTma) {  // TMA-staged tiles of 32 x 4 faces
-    CUtensorMap tm;
     if (!tma_tile_map(e, md, dir, &tm)) return;  // pangu_set_flux_config checked tma_ok
     const long long nt = (long long)d.NB * na * ((m + 3) / 4) * ((i1 - i0 + 1 + 31) / 32);
     if (dir == 2)
@@ -3167,7 +3305,7 @@ int run_flux_dir(pangu_engine *e, const pangu_pack *md, int dir, int march, int 
     case PANGU_METRIC_CKS: launch_flux_opt<CKS>(e, md, dir, march, threads, s); break;
     default: launch_flux_opt<MINKOWSKI>(e, md, dir, march, threads, s); break;
   }
-  ++e->launches;
+  e->launches += dir == 1 && x1_rest_lanes(e->d) ? 2 : 1;
   return check_launch();
 }
 
