@@ -98,6 +98,7 @@ int pangu_engine_destroy(pangu_engine *e) {
   cudaFree(e->d_f2tab32);
   cudaFree(e->d_f1tab);
   cudaFree(e->d_f2tab);
+  cudaFree(e->d_f3tab);
   cudaFree(e->d_t2);
   cudaFree(e->d_origin);
   cudaFree(e->d_xdst);
@@ -152,7 +153,36 @@ int validate_mesh(const pangu_params &p, const pangu_mesh &m) {
 
 // Allocates an empty pool of `capacity` block slots for up to `max_jobs`
 // jobs with the block shape of e->m.
-int pool_init(pangu_engine *e, int capacity, int max_jobs) {
+// Tables of the CKS metric for an engine of one mesh (a pool's capacity is not all
+// in use): 1.7 KB a cell, about twice the job's own arrays, against some 1,500
+// FP64 operations per metric evaluation, eight evaluations a cell and stage. They
+// are kept while they take at most an eighth of the memory that is free; where
+// they do not fit the kernels evaluate the metric, to the same bits.
+void cks_tables(pangu_engine *e) {
+  const Dims &d = e->d;
+  constexpr TabLayout T = tab_layout(CKS);
+  const size_t c = e->capacity;
+  const size_t n[4] = {c * d.N3 * d.N2 * tab_row(d.N1, T.ncen),
+                       c * d.N3 * d.N2 * tab_row(d.N1 + 1, T.nmet),
+                       c * d.N3 * (d.N2 + 1) * tab_row(d.N1, T.nmet),
+                       c * (d.N3 + 1) * d.N2 * tab_row(d.N1, T.nmet)};
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+      (n[0] + n[1] + n[2] + n[3]) * sizeof(double) > free_b / 8)
+    return;
+  double **t[4] = {&e->d_ctab, &e->d_f1tab, &e->d_f2tab, &e->d_f3tab};
+  bool ok = true;
+  for (int q = 0; q < 4; ++q) ok = ok && dalloc(t[q], n[q]) == PANGU_OK;
+  if (!ok) {
+    cudaGetLastError();  // an allocation that failed is no error of the engine
+    for (int q = 0; q < 4; ++q) {
+      cudaFree(*t[q]);
+      *t[q] = nullptr;
+    }
+  }
+}
+
+int pool_init(pangu_engine *e, int capacity, int max_jobs, bool one_mesh) {
   const pangu_params &p = e->p;
   pangu_mesh one = e->m;
   one.nbx1 = one.nbx2 = one.nbx3 = 1;
@@ -225,6 +255,7 @@ int pool_init(pangu_engine *e, int capacity, int max_jobs) {
     }
   }
   if (rc != PANGU_OK) return PANGU_ENOMEM;
+  if (p.metric_type == PANGU_METRIC_CKS && one_mesh) cks_tables(e);
   bool ok = cudaMemset(e->d_cnt, 0, (size_t)max_jobs * PANGU_NCOUNTERS * 8) == cudaSuccess;
   ok &= cudaMemset(e->d_slot_job, 0, (size_t)capacity * sizeof(int)) == cudaSuccess;
   ok &= cudaMemset(e->d_bcf, 0xff, 6 * (size_t)capacity) == cudaSuccess;  // -1: no BC
@@ -246,6 +277,7 @@ int pool_init(pangu_engine *e, int capacity, int max_jobs) {
   d.f2tab32 = e->d_f2tab32;
   d.f1tab = e->d_f1tab;
   d.f2tab = e->d_f2tab;
+  d.f3tab = e->d_f3tab;
   return PANGU_OK;
 }
 
@@ -413,6 +445,20 @@ int pool_attach(pangu_engine *e, const pangu_mesh &m, double a, double h, int *j
     }
     if (!ok) return PANGU_ECUDA;
   }
+  if (e->p.metric_type == PANGU_METRIC_CKS && e->d_ctab) {
+    ok = cudaMemcpy(e->d_tmp_slots, slots.data(), slots.size() * sizeof(int),
+                    cudaMemcpyHostToDevice) == cudaSuccess;
+    Dims dj = d;
+    dj.slot = e->d_tmp_slots;
+    dj.NB = (int)nbl;
+    double *tabs[4] = {e->d_ctab, e->d_f1tab, e->d_f2tab, e->d_f3tab};
+    for (int kind = 0; kind < 4 && ok; ++kind)
+      k_build_tables_cks<<<grid_for((long long)dj.NB * (d.N3 + (kind == 3)) * (d.N2 + (kind == 2)) *
+                                    (d.N1 + (kind == 1))),
+                           kThreads>>>(dj, J.p, kind, tabs[kind]);
+    ok = ok && cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
+    if (!ok) return PANGU_ECUDA;
+  }
   J.live = true;
   for (int sl : slots) e->slot_used[sl] = 1;
   e->jobs[job] = std::move(J);
@@ -450,7 +496,7 @@ int pangu_engine_create(const pangu_params *params, const pangu_mesh *mesh, pang
   e->p = *params;
   e->m = *mesh;
   const int nb = mesh->nbx1 * mesh->nbx2 * mesh->nbx3;
-  rc = pool_init(e, nb, 1);
+  rc = pool_init(e, nb, 1, true);
   int job = -1;
   if (!rc) rc = pool_attach(e, *mesh, params->a, params->h, &job, nullptr);
   if (rc) {
@@ -472,7 +518,7 @@ int pangu_pool_create(const pangu_params *params, const pangu_mesh *block, int32
   if (!e) return PANGU_ENOMEM;
   e->p = *params;
   e->m = *block;
-  rc = pool_init(e, capacity_blocks, max_jobs);
+  rc = pool_init(e, capacity_blocks, max_jobs, false);
   if (rc) {
     pangu_engine_destroy(e);
     return rc;
@@ -686,7 +732,7 @@ int pangu_shard_create(const pangu_params *params, const pangu_mesh *mesh,
   e->m = *mesh;
   e->nranks = nranks;
   e->rank = rank;
-  rc = pool_init(e, nloc, 1);
+  rc = pool_init(e, nloc, 1, true);
   int job = -1;
   if (!rc) rc = pool_attach(e, *mesh, params->a, params->h, &job, nullptr, block_rank);
   if (rc) {

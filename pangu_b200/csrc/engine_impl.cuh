@@ -59,8 +59,9 @@ struct Dims {
   // Static MKS/BL metric tables (built once per engine by k_build_tables):
   // N2 x N1 points per slot at the centres, N2 x (N1 + 1) at the x1 faces and
   // (N2 + 1) x N1 at the x2 faces, laid out by tab_at (kernels.cuh); x3 faces use
-  // the centres.
-  const double *ctab, *f1tab, *f2tab;
+  // the centres. CKS engines (where they fit): N3 N2 rows of N1 cells, and the
+  // faces of all three directions.
+  const double *ctab, *f1tab, *f2tab, *f3tab;
   // Mixed form only: the centre table rounded once to FP32, read by the FP32
   // source term, electron heating and the x3 faces; null otherwise.
   const float *ctab32;
@@ -109,7 +110,7 @@ struct pangu_engine {
   double *d_bdx = nullptr;      // [capacity][3]
   signed char *d_bcf = nullptr; // [capacity][6]
   double *d_t1 = nullptr, *d_t2 = nullptr, *d_origin = nullptr;
-  double *d_ctab = nullptr, *d_f1tab = nullptr, *d_f2tab = nullptr;
+  double *d_ctab = nullptr, *d_f1tab = nullptr, *d_f2tab = nullptr, *d_f3tab = nullptr;
   float *d_ctab32 = nullptr;  // mixed form: FP32 centre table
   float *d_f1tab32 = nullptr, *d_f2tab32 = nullptr;  // mixed form: FP32 face tables
   long long *d_xdst = nullptr, *d_xsrc = nullptr;  // [capacity x ghost cells per block]

@@ -202,6 +202,10 @@ __device__ __forceinline__ void gcov_at(const Dims &d, const pangu_params &p, in
 // structurally non-zero Christoffel symbols (symmetric in their lower
 // indices). Loads reproduce the dense values bit for bit.
 // ---------------------------------------------------------------------------
+// The CKS metric depends on all three coordinates: its tables hold every entry of
+// every cell and face (gcov and the connection unsymmetric, as the dense
+// arithmetic leaves them) and exist where they fit (cks_tables in engine.cu);
+// otherwise the kernels form the metric at each point.
 struct TabLayout {
   int nsym, ncon, nmet, nconn, ncen;
   int sym[4][4];      // slot of g_rc (r, c symmetric), -1 if structurally zero
@@ -215,11 +219,12 @@ __host__ __device__ constexpr TabLayout tab_layout(int mt) {
   int n = 0;
   for (int r = 0; r < 4; ++r)
     for (int c = 0; c < 4; ++c) L.sym[r][c] = -1;
+  const bool full = mt == CKS;  // xi l_r l_c and xi l_c l_r round differently
   for (int r = 0; r < 4; ++r)
-    for (int c = r; c < 4; ++c)
+    for (int c = full ? 0 : r; c < 4; ++c)
       if (pt.nz[r][c]) {
         L.sym[r][c] = n;
-        L.sym[c][r] = n;
+        if (!full) L.sym[c][r] = n;
         ++n;
       }
   L.nsym = n;
@@ -241,13 +246,13 @@ __host__ __device__ constexpr TabLayout tab_layout(int mt) {
       for (int k = 0; k < 4; ++k) L.conn[a][j][k] = -1;
   for (int a = 0; a < 4; ++a)
     for (int j = 0; j < 4; ++j)
-      for (int k = j; k < 4; ++k) {
+      for (int k = full ? 0 : j; k < 4; ++k) {
         bool nz = false;
         for (int l = 0; l < 4; ++l)
           nz = nz || (pt.nz[a][l] && (dg[j][l][k] || dg[k][l][j] || dg[l][j][k]));
         if (nz) {
           L.conn[a][j][k] = m;
-          L.conn[a][k][j] = m;
+          if (!full) L.conn[a][k][j] = m;
           ++m;
         }
       }
@@ -339,6 +344,25 @@ __device__ __forceinline__ int analytic_geo(const Dims &d, const pangu_params &p
   return ok;
 }
 
+// analytic_geo of the CKS metric out of line, for engines without its tables.
+__device__ __noinline__ int cks_geo(double x, double y, double z, double a, Geo *o) {
+  Geo g;
+  cks_code_gcov(x, y, z, a, g.gcov);
+  const int ok = gj_invert(g.gcov, g.gcon);
+  g.gdet = determinant(g.gcov);
+  g.sg = sqrt(fabs(g.gdet));
+  g.alpha = 1.0 / sqrt(-g.gcon[0][0]);
+  *o = g;
+  return ok;
+}
+__device__ __forceinline__ int cks_geo_at(const pangu_params &p, double x, double y, double z,
+                                          Geo &g) {
+  Geo c;
+  const int ok = cks_geo(x, y, z, p.a, &c);
+  g = c;
+  return ok;
+}
+
 // ComputeMetricAtLocation (christoffel.h:53-62) at cell centre (b, k, j, i).
 // Returns 0 if the metric is singular.
 template <int MT>
@@ -348,8 +372,11 @@ __device__ __forceinline__ int cell_metric(const Dims &d, const pangu_params &p,
     constexpr TabLayout L = tab_layout(MT);
     return load_geo<MT>(d.ctab + tab_at(L.ncen, d.N2, d.N1, b, j, i), g);
   } else if (MT == CKS) {
-    const double x[4] = {0.0, xc(d, b, 0, i), xc(d, b, 1, j), xc(d, b, 2, k)};
-    return analytic_geo<MT>(d, p, b, i, 0, j, 0, x, g);
+    if (d.ctab) {
+      constexpr TabLayout L = tab_layout(MT);
+      return load_geo<MT>(d.ctab + tab_at(L.ncen, d.N3 * d.N2, d.N1, b, k * d.N2 + j, i), g);
+    }
+    return cks_geo_at(p, xc(d, b, 0, i), xc(d, b, 1, j), xc(d, b, 2, k), g);
   } else {
     minkowski_geo(g);
     return 1;
@@ -385,10 +412,17 @@ __device__ __forceinline__ int face_metric(const Dims &d, const pangu_params &p,
       return load_geo<MT>(d.f2tab + tab_at(L.nmet, d.N2 + 1, d.N1, b, j, i), g);
     return cell_metric<MT>(d, p, b, k, j, i, g);  // independent of x3
   } else if (MT == CKS) {
-    const double x[4] = {0.0, dir == 1 ? xf(d, b, 0, i) : xc(d, b, 0, i),
-                         dir == 2 ? xf(d, b, 1, j) : xc(d, b, 1, j),
-                         dir == 3 ? xf(d, b, 2, k) : xc(d, b, 2, k)};
-    return analytic_geo<MT>(d, p, b, i, 0, j, 0, x, g);
+    if (d.ctab) {
+      constexpr TabLayout L = tab_layout(MT);
+      const double *t =
+          dir == 1 ? d.f1tab + tab_at(L.nmet, d.N3 * d.N2, d.N1 + 1, b, k * d.N2 + j, i)
+          : dir == 2 ? d.f2tab + tab_at(L.nmet, d.N3 * (d.N2 + 1), d.N1, b, k * (d.N2 + 1) + j, i)
+                     : d.f3tab + tab_at(L.nmet, (d.N3 + 1) * d.N2, d.N1, b, k * d.N2 + j, i);
+      return load_geo<MT>(t, g);
+    }
+    return cks_geo_at(p, dir == 1 ? xf(d, b, 0, i) : xc(d, b, 0, i),
+                      dir == 2 ? xf(d, b, 1, j) : xc(d, b, 1, j),
+                      dir == 3 ? xf(d, b, 2, k) : xc(d, b, 2, k), g);
   } else {
     minkowski_geo(g);
     return 1;
@@ -2104,10 +2138,13 @@ __device__ __forceinline__ void source_cell(const Dims &d, const pangu_params &p
   double T[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) emt_from_state(p.adiabatic_index, pc, s, r, T[r]);
-  if (MT == MKS || MT == BL) {
+  if (MT == MKS || MT == BL || (MT == CKS && d.ctab)) {
     // Christoffel symbols from the centre table; structural zeros skipped
     constexpr TabLayout L = tab_layout(MT);
-    const double *cn = d.ctab + tab_at(L.ncen, d.N2, d.N1, b, j, i) + L.nmet * kTabCols;
+    const double *cn =
+        d.ctab + L.nmet * kTabCols +
+        (MT == CKS ? tab_at(L.ncen, d.N3 * d.N2, d.N1, b, k * d.N2 + j, i)
+                   : tab_at(L.ncen, d.N2, d.N1, b, j, i));
     // the four contractions first, then the four updates: no Christoffel load
     // waits behind a store to U
     double con[4];
@@ -2222,6 +2259,51 @@ __global__ void __launch_bounds__(kThreads) k_build_tables(Dims d, pangu_params 
 #pragma unroll
         for (int kk = jj; kk < 4; ++kk)
           if (L.conn[a][jj][kk] >= 0) o[(L.nmet + L.conn[a][jj][kk]) * plane] = conn[a][jj][kk];
+  }
+}
+
+// The same for a CKS engine: centres (kind 0) or the faces of direction `kind`,
+// one launch each.
+__global__ void __launch_bounds__(kThreads) k_build_tables_cks(Dims d, pangu_params p, int kind,
+                                                               double *tab) {
+  pdl_grid_wait();
+  constexpr TabLayout L = tab_layout(CKS);
+  const int W = d.N1 + (kind == 1), R2 = d.N2 + (kind == 2), R3 = d.N3 + (kind == 3);
+  const int nc = kind == 0 ? L.ncen : L.nmet;
+  const long long per = (long long)R3 * R2 * W;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= per * d.NB) return;
+  long long q, kj, il, jl;
+  const int b = slot_of(d, (int)div_fast(t, per, q));
+  kj = div_fast(q, W, il);
+  const int k = (int)div_fast(kj, R2, jl), j = (int)jl, i = (int)il;
+  const double x = kind == 1 ? xf(d, b, 0, i) : xc(d, b, 0, i),
+               y = kind == 2 ? xf(d, b, 1, j) : xc(d, b, 1, j),
+               z = kind == 3 ? xf(d, b, 2, k) : xc(d, b, 2, k);
+  Geo g;
+  const int ok = cks_geo_at(p, x, y, z, g);
+  double *o = tab + tab_at(nc, R3 * R2, W, b, (int)kj, i);
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      o[L.sym[r][c] * kTabCols] = g.gcov[r][c];
+      o[(L.nsym + L.con[r][c]) * kTabCols] = g.gcon[r][c];
+    }
+  constexpr int s0 = L.nsym + L.ncon;
+  o[s0 * kTabCols] = g.gdet;
+  o[(s0 + 1) * kTabCols] = g.sg;
+  o[(s0 + 2) * kTabCols] = g.alpha;
+  o[(s0 + 3) * kTabCols] = ok ? 1.0 : 0.0;
+  if (kind == 0) {
+    double conn[4][4][4];
+    christoffel<CKS>(d, p, b, k, j, i, g, conn);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) o[(L.nmet + L.conn[a][jj][kk]) * kTabCols] = conn[a][jj][kk];
   }
 }
 
