@@ -50,13 +50,15 @@ __host__ __forceinline__ PT *prim_of(const Pack *md) {
   return reinterpret_cast<PT *>(md->prim);
 }
 
-// CTA size of the per-cell kernels. FixPrimitive, the geometric source and
-// electron heating are bounded to 4 resident CTAs per SM (64 registers): the
-// extra occupancy outweighs their few spills (measured 2 % per RK2 cycle on
-// the 2D and 3D tori), and 148 x 1024 threads hold a 512 x 256 grid in one
-// wave. The first C2P pass runs in CTAs of 128 threads bounded to 7 per SM
-// (72 registers, a few spills): 148 x 896 threads hold the 512 x 256 grid in
-// one wave (1.2 % per cycle; at 64 registers its Newton loop spills too much).
+// CTA size of the per-cell kernels. The geometric source and electron heating are
+// bounded to 4 resident CTAs per SM (64 registers): the extra occupancy outweighs
+// their few spills (measured 2 % per RK2 cycle on the 2D and 3D tori), and
+// 148 x 1024 threads hold a 512 x 256 grid in one wave. FixPrimitive forms its
+// state once and stores the conserved variables before its powers; bound by issue
+// and FP64 latency, it runs best in CTAs of 128 bounded to 6 per SM (80
+// registers): 742 us per cycle on the 3D torus, 953 at 64 registers, 852 at 128,
+// and 794 for the form with a second state. The first C2P pass runs in CTAs of
+// 128 threads bounded to 7 per SM (72 registers), its chained form to 6.
 constexpr int kThreads = 256;
 constexpr int kRecoveryThreads = 128;
 constexpr int kFixThreads = 128;
@@ -266,7 +268,8 @@ __host__ __device__ constexpr TabLayout tab_layout(int mt) {
 // lie a constant 128 bytes apart, so that a thread forms one address and every
 // load takes its component as an immediate offset (a plane per component cost
 // two or three integer instructions a load), and a warp's 32 columns read whole
-// 128-byte lines as before.
+// 128-byte lines as before. Per cycle of the 3D torus: staged x2 and x3 fluxes
+// 3022 against 3154 us, FP32 source term 273 against 333 us.
 constexpr int kTabCols = 16;
 __host__ __device__ constexpr long long tab_row(int W, int nc) {
   return (long long)((W + kTabCols - 1) / kTabCols) * kTabCols * nc;
@@ -385,7 +388,8 @@ __device__ __forceinline__ int cell_metric(const Dims &d, const pangu_params &p,
 
 #if PGK_MIXED
 // cell_metric rounded to FP32: from the FP32 copy of the centre table (half the
-// bytes and no conversions), or cast.
+// bytes and no conversions; x3 faces 727 against 765 us per cycle on the 3D
+// torus), or cast.
 template <int MT>
 __device__ __forceinline__ int cell_metric_f32(const Dims &d, const pangu_params &p, int b, int k,
                                                int j, int i, GeoT<FT> &g) {
@@ -997,21 +1001,26 @@ __device__ __forceinline__ void face_side(double gam, const double P[NPRIM], con
 template <int c>
 __device__ __forceinline__ FT flux_component_t(FT gam, const FT P[NPRIM], const StateT<FT> &s,
                                                FT sg, int dir) {
-  const FT f_rho = P[RHO] * s.ucon[dir];
-  if (c == RHO) return f_rho * sg;
-  if (c == ENT) return (P[ENT] * f_rho) * sg;
-  if (c == KEL) return (P[KEL] * f_rho) * sg;
+  const FT f_rho = tmul(P[RHO], s.ucon[dir]);
+  if (c == RHO) return tmul(f_rho, sg);
+  if (c == ENT) return tmul(tmul(P[ENT], f_rho), sg);
+  if (c == KEL) return tmul(tmul(P[KEL], f_rho), sg);
   if (c >= BX1 && c <= BX3) {
     const int m = c - BX1 + 1;
-    return (s.bcon[m] * s.ucon[dir] - s.bcon[dir] * s.ucon[m]) * sg;
+    return tmul(tdot2(s.bcon[m], s.ucon[dir], -s.bcon[dir], s.ucon[m]), sg);
   }
-  const FT hh = P[RHO] + gam * P[ENY];
-  const FT e_tot = hh + s.bsq;
-  const FT p_tot = (gam - FT(1)) * P[ENY] + FT(0.5) * s.bsq;
+  const FT e_tot = tadd(tfma(gam, P[ENY], P[RHO]), s.bsq);
   const int m = (c == ENY) ? 0 : c - UX1 + 1;
-  const FT t = e_tot * s.ucon[dir] * s.ucov[m] + p_tot * FT(dir == m) - s.bcon[dir] * s.bcov[m];
-  if (c == ENY) return (t + f_rho) * sg;
-  return t * sg;
+  const FT eu = tmul(e_tot, s.ucon[dir]);
+  FT t;
+  if (dir == m) {
+    const FT p_tot = tfma(FT(0.5), s.bsq, tmul(tadd(gam, FT(-1)), P[ENY]));
+    t = tfma(-s.bcon[dir], s.bcov[m], tfma(eu, s.ucov[m], p_tot));
+  } else {
+    t = tdot2(eu, s.ucov[m], -s.bcon[dir], s.bcov[m]);
+  }
+  if (c == ENY) return tmul(tfma(P[RHO], s.ucon[dir], t), sg);
+  return tmul(t, sg);
 }
 
 // Riemann flux and fast speed at the lower face of (b, k, j, i) along DIR in
@@ -1055,16 +1064,17 @@ __device__ __forceinline__ void face_flux(const Dims &d, const pangu_params &p, 
   const FT cms = tmax(cmax, cmin);
   a_alfven(d, alfven, b, DIR - 1)[fo] = cms;
   const bool hll = PGK_FLUX_HLL(p);
-  const FT ihll = FT(1) / (cmax + cmin + FT(1e-20));
+  const FT ihll = FT(1) / (cmax + cmin + FT(1e-20)), cmm = tmul(cmax, cmin);
 #define PGD_FACE_COMPONENT(C)                                                         \
   if (d.pidx[C] >= 0) {                                                               \
     const FT fl = flux_component_t<C>(gam, PL, sL, sg, DIR);                          \
     const FT fr = flux_component_t<C>(gam, PR, sR, sg, DIR);                          \
     const FT ul = flux_component_t<C>(gam, PL, sL, sg, 0);                            \
     const FT ur = flux_component_t<C>(gam, PR, sR, sg, 0);                            \
-    a_flux(d, F, b, d.pidx[C])[fo] =                                                     \
-        hll ? (cmax * fl + cmin * fr - cmax * cmin * (ur - ul)) * ihll                 \
-            : FT(0.5) * (fl + fr - cms * (ur - ul));                                   \
+    const FT du = tadd(ur, -ul);                                                      \
+    a_flux(d, F, b, d.pidx[C])[fo] =                                                  \
+        hll ? tmul(tfma(-cmm, du, tdot2(cmax, fl, cmin, fr)), ihll)                    \
+            : tmul(FT(0.5), tfma(-cms, du, tadd(fl, fr)));                             \
   }
   PGD_FACE_COMPONENT(RHO)
   PGD_FACE_COMPONENT(ENY)
@@ -1247,7 +1257,8 @@ constexpr int kFluxBlocks = 4;
 // The mixed form's tabulated-metric kernels need 72 registers with one face's
 // reconstruction in flight and 96 with a march; bounds that say so keep ptxas
 // from taking 80 and 108 (x1 947 against 1052 us per cycle on the 3D torus, x2
-// and x3 1576 against 1758).
+// and x3 1576 against 1758). Their arithmetic is spelled out, so the bound
+// changes no result.
 constexpr int flux_blocks(int mt, bool march) {
   return !PGK_MIXED || mt == CKS ? kFluxBlocks : (march ? 5 : 7);
 }
@@ -1584,8 +1595,8 @@ __device__ __forceinline__ bool tma_wait(unsigned long long *bar, int *err) {
 
 // x2 / x3 faces: tiles of 32 x TF faces. The copy holds the tile's 32 columns
 // (plus the few that align its start) and the TF + 5 cells along the face
-// direction that the TF faces' stencils reach; each thread reconstructs the
-// two cells of its face.
+// direction that the TF faces' stencils reach. PPM4's face values are formed once
+// for the tile, then each thread limits the two cells of its face.
 constexpr int kTmaCols = 32 + kTmaAlign;
 
 // Bytes of the staged primitives.
@@ -1901,13 +1912,9 @@ __global__ void __launch_bounds__(kThreads) k_ct_faces(Dims d, double *F1, doubl
 // block's widths, areas, volume and beta dt are formed once per cell, not once
 // per (cell, variable) (4x fewer instructions; every variable's value is
 // computed as before).
-__global__ void __launch_bounds__(kThreads, 4) k_flux_div_update(Dims d, const double *F1,
-                                                                 const double *F2,
-                                                                 const double *F3,
-                                                                 const double *Uinit,
-                                                                 double *Uout, double beta,
-                                                                 const double *dt) {
-  pdl_grid_wait();
+__device__ __forceinline__ void update_cell(const Dims &d, const double *F1, const double *F2,
+                                            const double *F3, const double *Uinit, double *Uout,
+                                            double beta, const double *dt) {
   int b, k, j, i;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (!box_index(t, d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie, b, k, j, i)) return;
@@ -1959,15 +1966,22 @@ __global__ void __launch_bounds__(kThreads, 4) k_flux_div_update(Dims d, const d
     }
   }
 }
+__global__ void __launch_bounds__(kThreads, 4) k_flux_div_update(Dims d, const double *F1,
+                                                                 const double *F2,
+                                                                 const double *F3,
+                                                                 const double *Uinit,
+                                                                 double *Uout, double beta,
+                                                                 const double *dt) {
+  pdl_grid_wait();
+  update_cell(d, F1, F2, F3, Uinit, Uout, beta, dt);
+}
 
 // ---------------------------------------------------------------------------
 // Ghost exchange: ghost <- neighbour interior, prim and flag.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_exchange(Dims d, long long n, const long long *dst,
-                                                       const long long *src, PT *P,
-                                                       double *flag) {
-  pdl_grid_wait();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void exchange_cell(const Dims &d, long long t, long long n,
+                                              const long long *dst, const long long *src, PT *P,
+                                              double *flag) {
   if (t >= n) return;
   const long long dc = dst[t], sc = src[t];
   long long db, dof, sb, sof;
@@ -1985,6 +1999,31 @@ __global__ void __launch_bounds__(kThreads) k_exchange(Dims d, long long n, cons
   for (int v = 0; v < NPRIM; ++v)
     if (v < d.NF) a_prim(d, P, (int)db, v)[dof] = val[v];
   if (has_flag) a_flag(d, flag, (int)db)[dof] = fl;
+}
+
+__global__ void __launch_bounds__(kThreads) k_exchange(Dims d, long long n, const long long *dst,
+                                                       const long long *src, PT *P,
+                                                       double *flag) {
+  pdl_grid_wait();
+  exchange_cell(d, (long long)blockIdx.x * blockDim.x + threadIdx.x, n, dst, src, P, flag);
+}
+
+// FluxDivergence + UpdateIndependentData and, in the CTAs from nu on, the ghost
+// exchange that follows them in a stage: the update writes conserved variables
+// from the fluxes, the exchange copies primitives and flags, so neither waits for
+// the other and a stage has a launch less (3 to 4 us of the 256^2 vortex's 55).
+// dx: the Dims of the exchanged container.
+__global__ void __launch_bounds__(kThreads, 4)
+    k_update_exchange(Dims d, const double *F1, const double *F2, const double *F3,
+                      const double *Uinit, double *Uout, double beta, const double *dt,
+                      unsigned nu, Dims dx, long long n, const long long *dst,
+                      const long long *src, PT *P, double *flag) {
+  pdl_grid_wait();
+  if (blockIdx.x < nu)
+    update_cell(d, F1, F2, F3, Uinit, Uout, beta, dt);
+  else
+    exchange_cell(dx, (long long)(blockIdx.x - nu) * blockDim.x + threadIdx.x, n, dst, src, P,
+                  flag);
 }
 
 // Halo messages of a sharded mesh: the cells of the exchange whose other end
@@ -2445,12 +2484,17 @@ __device__ __forceinline__ void c2p_write(const Dims &d, PT *P, int b, int k, in
 // cells. CHAIN = true: the failing lanes run Scheme1Dvsq and Scheme1D at
 // once (the retry pass's arithmetic, from the same inputs), and `list` (may
 // be null) receives the cells the whole chain fails, FixRecovery's list.
-// The chained form is used when the pass fits in one wave of CTAs: then the
+// The chained form is used when the pass has at most 7 CTAs per SM: then the
 // few long chains overlap the rest of the wave instead of running as a
 // separate latency-bound launch (2D 512 x 256 torus at steady state: 0.387
 // against 0.403 ms per cycle), while on larger grids the registers the
 // chain adds (spills) cost more than the retry launch (3D torus 11.17
 // against 10.98 ms, 48-torus batch 7.15 against 7.05 ms).
+// Bound by the latency of the Newton steps' dependent FP64 operations. With the
+// steps' divisions branch-free (newton_2d_step), per cycle: 718 against 819 us on
+// the 3D torus (667 against 773 in the mixed form), the chained form 59.6 against
+// 63.4 us on the 2D torus at 6 CTAs per SM (61 at 5, 61.8 at 7). Bounds of 6 and
+// 5 on the plain form: 814 us and no change.
 // (Folding the geometric source and electron heating into this kernel was
 // measured slower: their registers cut the occupancy of the Newton loops.)
 template <int MT, bool CHAIN>
@@ -2600,12 +2644,21 @@ __global__ void __launch_bounds__(kThreads) k_fixrec_scan(Dims d, pangu_params p
   list[n] = fc;
 }
 
-__global__ void __launch_bounds__(kThreads) k_fixrec_compute(Dims d, const int *count_in,
-                                                             const long long *list,
-                                                             const PT *P, const double *flag,
-                                                             double *vals) {
+// Both phases in one launch: every CTA computes the values of its cells from the
+// primitives and flags as they stand; the CTA that finishes last (a ticket taken
+// after a fence, no waiting) writes them all. Nothing fails in most stages, and a
+// launch that finds the list empty costs 3 us of a cycle's 70 to 300, so one
+// launch instead of two; the last CTA's 1024 threads write a thousand cells in
+// about 2 us.
+constexpr int kFixRecThreads = 1024;
+__global__ void __launch_bounds__(kFixRecThreads) k_fixrec(Dims d, const int *count_in,
+                                                           const long long *list, PT *P,
+                                                           double *flag, double *vals,
+                                                           unsigned long long *cnt,
+                                                           unsigned int *ticket) {
   pdl_grid_wait();
   const int n = *count_in;
+  if (n == 0) return;
   const int off2 = d.js != d.je ? 1 : 0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -2630,30 +2683,28 @@ __global__ void __launch_bounds__(kThreads) k_fixrec_compute(Dims d, const int *
       vals[t * d.NF + v] = val;
     }
   }
-}
-
-__global__ void __launch_bounds__(kThreads) k_fixrec_write(Dims d, const int *count_in,
-                                                           const long long *list,
-                                                           const double *vals, PT *P,
-                                                           double *flag,
-                                                           unsigned long long *cnt) {
-  pdl_grid_wait();
-  const int n = *count_in;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
     const long long fc = list[t];
     const long long b = fc / d.ncell;
     const long long c = fc - b * d.ncell;
     double w[NPRIM];
 #pragma unroll
     for (int v = 0; v < NPRIM; ++v)
-      if (v < d.NF) w[v] = vals[t * d.NF + v];
+      if (v < d.NF) w[v] = __ldcg(vals + (long long)t * d.NF + v);  // other CTAs' stores: past L1
 #pragma unroll
     for (int v = 0; v < NPRIM; ++v)
       if (v < d.NF) a_prim(d, P, (int)b, v)[c] = (v >= 2 && v < 5) ? PT(0) : (PT)w[v];
     a_flag(d, flag, (int)b)[c] = 1;
     count(cnt, job_of(d, (int)b), PANGU_CNT_FIXRECOVERY, true);
   }
+  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -3249,17 +3300,17 @@ inline bool tma_tile_map(const pangu_engine *e, const pangu_pack *md, int dir, C
 
 // Lanes per row of k_flux_x1_rest, or 0 where the x1 kernel takes every face: a
 // row of nf faces fills nf / 31 warps and leaves nf % 31 faces, which as a
-// segment of their own cost a whole warp. Packed, they cost G / 32 of one and a
-// launch; worth it where the warps saved fill the GPU once (16 per SM, about
-// 15 us of x1 work, against 2 to 4 us for a launch). 64^3 blocks have 65 faces:
-// 2.1 warps a row for 3 (x1 XXX against YYY us per cycle on the 3D torus), 32^3
-// blocks 33: 1.1 for 2.
+// segment of their own cost a whole warp. Up to three are packed, 8 or 16 rows to
+// a warp, where the warps saved fill the GPU once (16 per SM, about 15 us of x1
+// work, against 2 to 4 us for a launch). 64^3 blocks have 65 faces: 2.1 warps a
+// row for 3 (x1 1414 against 1642 us per cycle on the 3D torus), 32^3 blocks 33:
+// 1.1 for 2. Groups of 8 lanes lost what they saved to their short loads (252
+// against 237 us on twelve tori in blocks of 128 x 64).
 inline int x1_rest_lanes(const Dims &d) {
   const int nf = d.ie + 1 - d.is + 1, rest = nf % kFacesPerWarp;
   if (rest == 0 || nf < kFacesPerWarp) return 0;
-  int G = 2;
-  while (G < rest + 1) G *= 2;
-  if (G > 16) return 0;
+  if (rest > 3) return 0;
+  const int G = rest == 1 ? 2 : 4;
   const long long rows = (long long)d.NB * (d.ke - d.ks + 1 + 2 * d.o3) * (d.je - d.js + 1 + 2 * d.o2);
   return rows * (32 - G) / 32 >= 16LL * device_sms() ? G : 0;
 }
@@ -3475,6 +3526,8 @@ int run_ct(pangu_engine *e, const pangu_pack *md, cudaStream_t s) {
   return check_launch();
 }
 
+int run_exchange(pangu_engine *e, const pangu_pack *md, cudaStream_t s);
+
 int run_update(pangu_engine *e, const pangu_pack *mi, const pangu_pack *m0, const pangu_pack *m1,
                double beta, const double *dt, cudaStream_t s) {
   Dims d = bind(e, m0);  // the fluxes of mc0
@@ -3483,6 +3536,26 @@ int run_update(pangu_engine *e, const pangu_pack *mi, const pangu_pack *m0, cons
   const long long n = box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie);
   launch_pdl(k_flux_div_update, dim3(grid_for(n)), dim3(kThreads), s, d, m0->flux1, m0->flux2,
              m0->flux3, mi->cons, m1->cons, beta, dt);
+  ++e->launches;
+  return check_launch();
+}
+
+// The update with the exchange of mc1's ghosts in the same launch.
+int run_update_exchange(pangu_engine *e, const pangu_pack *mi, const pangu_pack *m0,
+                        const pangu_pack *m1, double beta, const double *dt, cudaStream_t s) {
+  if (e->nxch == 0) return run_update(e, mi, m0, m1, beta, dt, s);
+  Dims d = bind(e, m0);
+  d.tU = m1->cons_vars;
+  d.tUi = mi->cons_vars;
+  const unsigned nu = grid_for(box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie));
+  const unsigned nx = grid_for(e->nxch);
+  if ((long long)nu + nx > 0x7fffffffLL) {
+    const int rc = run_update(e, mi, m0, m1, beta, dt, s);
+    return rc ? rc : run_exchange(e, m1, s);
+  }
+  launch_pdl(k_update_exchange, dim3(nu + nx), dim3(kThreads), s, d, m0->flux1, m0->flux2,
+             m0->flux3, mi->cons, m1->cons, beta, dt, nu, bind(e, m1), e->nxch, e->d_xdst,
+             e->d_xsrc, prim_of(m1), m1->flag);
   ++e->launches;
   return check_launch();
 }
@@ -3586,12 +3659,9 @@ int run_fix_recovery(pangu_engine *e, const pangu_pack *md, bool listed, cudaStr
     k_fixrec_scan<<<grid_for(n), kThreads, 0, s>>>(d, e->p, md->flag, count, list);
     ++e->launches;
   }
-  const unsigned g = 2 * 148;
-  launch_pdl(k_fixrec_compute, dim3(g), dim3(kThreads), s, d, count, list, prim_of(md), md->flag,
-             e->d_fail_vals);
-  launch_pdl(k_fixrec_write, dim3(g), dim3(kThreads), s, d, count, list, e->d_fail_vals,
-             prim_of(md), md->flag, e->d_cnt);
-  e->launches += 2;
+  launch_pdl(k_fixrec, dim3(64), dim3(kFixRecThreads), s, d, count, list, prim_of(md), md->flag,
+             e->d_fail_vals, e->d_cnt, e->d_fix_ticket);
+  ++e->launches;
   return check_launch();
 }
 
@@ -3639,7 +3709,7 @@ int dalloc(T **p, size_t n) {
 // run_stage_update: FixPrimitive + CalculateConservative, fluxes, CT and the
 // update; reads only mc0 and mc_init, writes mc1's conserved variables.
 int run_stage_update(pangu_engine *e, int stage, const pangu_pack *base, const pangu_pack *one,
-                     double beta, const double *dt, cudaStream_t s) {
+                     double beta, const double *dt, bool exchange, cudaStream_t s) {
   const pangu_pack *mc0 = stage == 1 ? base : one;
   const pangu_pack *mc1 = stage == 1 ? one : base;
   int rc;
@@ -3657,21 +3727,28 @@ int run_stage_update(pangu_engine *e, int stage, const pangu_pack *base, const p
     if ((rc = run_ct(e, mc0, s))) return rc;
   }
   {
-    TaskRange r("FluxDivergence+UpdateIndependentData");
-    if ((rc = run_update(e, base, mc0, mc1, beta, dt, s))) return rc;
+    TaskRange r(exchange ? "FluxDivergence+UpdateIndependentData+GhostExchange"
+                         : "FluxDivergence+UpdateIndependentData");
+    if ((rc = exchange ? run_update_exchange(e, base, mc0, mc1, beta, dt, s)
+                       : run_update(e, base, mc0, mc1, beta, dt, s)))
+      return rc;
   }
   return PANGU_OK;
+}
+
+int run_stage_update(pangu_engine *e, int stage, const pangu_pack *base, const pangu_pack *one,
+                     double beta, const double *dt, cudaStream_t s) {
+  return run_stage_update(e, stage, base, one, beta, dt, false, s);
 }
 
 int run_stage_begin(pangu_engine *e, int stage, const pangu_pack *base, const pangu_pack *one,
                     double beta, const double *dt, double *send, cudaStream_t s) {
   const pangu_pack *mc1 = stage == 1 ? one : base;
-  int rc = run_stage_update(e, stage, base, one, beta, dt, s);
+  int rc = run_stage_update(e, stage, base, one, beta, dt, true, s);
   if (rc) return rc;
-  {
-    TaskRange r("GhostExchange");
-    if ((rc = run_exchange(e, mc1, s))) return rc;
-    if (send && (rc = run_halo_pack(e, mc1, send, s))) return rc;
+  if (send) {
+    TaskRange r("GhostExchange (halo)");
+    if ((rc = run_halo_pack(e, mc1, send, s))) return rc;
   }
   return PANGU_OK;
 }

@@ -1,0 +1,141 @@
+"""Branches of the stage kernels that a rule on sizes or options picks, at the
+sizes where they can go wrong, bit for bit against the CPU oracle: the packed
+last faces of x1 rows, fields too small for the branch-free quotients, electron
+heating with and without the state, FixRecovery's one launch, and the CKS metric
+tabulated or formed in the kernels."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+from parity_util import CASES, Case, field, to_device  # noqa: E402
+
+from pangu_b200 import abi  # noqa: E402
+from pangu_b200 import params as prm  # noqa: E402
+from pangu_b200 import problems  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(problem, extra, **kw):
+    CASES["_branch"] = (problem, kw, extra)
+    try:
+        return Case("_branch")
+    finally:
+        del CASES["_branch"]
+
+
+def _engine(case, hb):
+    from pangu_b200.engine import Engine
+    eng = Engine(case.params, case.mesh)
+    base, one = eng.new_containers()
+    to_device(hb, base)
+    return eng, base, one
+
+
+PPM4 = {("core", "limiter"): "ppm4", ("parthenon/mesh", "nghost"): 3}
+
+
+# faces per row nx + 1 = 31 m + rest: rest 1, 2, 3 are packed (groups of 2, 4 and 4
+# lanes), rest 0 and 4 are not; enough rows for the rule
+@pytest.mark.parametrize("nx,blocks", [(31, 16), (32, 16), (33, 16), (34, 16), (61, 12), (64, 12)])
+@pytest.mark.parametrize("limiter", ["mc", "ppm4"])
+def test_last_faces_of_x1_rows(nx, blocks, limiter):
+    over = {("core", "riemann_solver"): "hll"} if nx % 2 else {}
+    case = _case("ot", {**(PPM4 if limiter == "ppm4" else {}), **over}, n=nx * blocks, nblock=nx)
+    hb, _ = case.oracle_containers()
+    eng, db, _ = _engine(case, hb)
+    case.oracle.calculate_fluxes(hb)
+    for march in (1, 8):
+        if march == 8 and (nx + 2 * case.mesh.ng) % 2:
+            continue  # the staged kernels need rows of whole 16-byte units
+        eng.set_flux_config(x1_march=march)
+        db.flux1.zero_()
+        db.alfven.zero_()
+        eng.calculate_fluxes(db)
+        assert np.array_equal(field(db, "flux1"), hb.flux1), (nx, limiter, march)
+        assert np.array_equal(field(db, "alfven"), hb.alfven)
+
+
+@pytest.mark.parametrize("problem,kw,over", [
+    ("torus", dict(nx1=40, nx2=24), {}),
+    ("torus", dict(nx1=40, nx2=24, limiter="mc", riemann="hll"), {}),
+    ("ot", dict(n=32), {**PPM4, ("core", "riemann_solver"): "hll"})])
+def test_fields_down_to_the_smallest_numbers(problem, kw, over):
+    """The magnetic field of each cell scaled by 2^-e, e from 0 past the end of the
+    subnormal numbers, zeros of both signs among them."""
+    case = _case(problem, over, **kw)
+    hb, ho = case.oracle_containers()
+    rng = np.random.default_rng(5)
+    shape = hb.prim.shape[:1] + hb.prim.shape[2:]
+    scale = np.ldexp(rng.uniform(0.5, 1.0, shape), -rng.integers(0, 1100, shape))
+    scale[rng.random(shape) < 0.1] = -0.0
+    hb.prim[:, 5:8] = rng.uniform(-1.0, 1.0, hb.prim[:, 5:8].shape) * scale[:, None]
+    eng, db, do = _engine(case, hb)
+    to_device(ho, do)
+    dt = torch.full((1,), 1e-3, dtype=torch.float64, device="cuda")
+    for march, m2 in ((1, 1), (1, 0), (8, 8)):
+        eng.set_flux_config(x1_march=march, x2_march=m2)
+        case.oracle.calculate_fluxes(hb)
+        eng.calculate_fluxes(db)
+        for f in ("flux1", "flux2", "alfven"):
+            assert np.array_equal(field(db, f), getattr(hb, f)), (march, f)
+    case.oracle.stage(1, hb, ho, 0.5, 1e-3)
+    eng.stage(1, db, do, 0.5, dt)
+    for f in ("prim", "cons"):
+        assert np.array_equal(field(do, f), getattr(ho, f), equal_nan=True), f
+
+
+@pytest.mark.parametrize("model", sorted(abi.HEATING_MODEL))
+@pytest.mark.parametrize("suppress", [False, True])
+def test_heating_with_and_without_the_state(model, suppress):
+    case = _case("torus", {("electron", "model"): model,
+                           ("electron", "suppress_highb_heat"): suppress}, nx1=40, nx2=24)
+    hb, ho = case.oracle_containers()
+    case.oracle.stage(1, hb, ho, 0.5, 1e-3)
+    rng = np.random.default_rng(6)
+    ho.cons[:, 8:10] *= rng.uniform(0.5, 2.0, ho.cons[:, 8:10].shape)
+    eng, _, do = _engine(case, hb)
+    to_device(ho, do)
+    case.oracle.apply_electron_heating(ho)
+    eng.apply_electron_heating(do)
+    # the oracle's exp and log are the C library's: two ulp in the models that call them
+    a, b = field(do, "prim"), ho.prim
+    if model in ("howes", "kawazura", "rowan"):
+        np.testing.assert_allclose(a, b, rtol=1e-14, atol=0.0)
+    else:
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("share", [0.0, 1e-4, 0.02, 0.6, 1.0])
+def test_fix_recovery_of_any_number_of_cells(share):
+    case = Case("ot_mc_laxf") if share < 0.5 else _case("ot", {}, n=288)
+    hb, _ = case.oracle_containers()
+    rng = np.random.default_rng(7)
+    hb.flag[...] = (rng.random(hb.flag.shape) >= share).astype(float)
+    eng, db, _ = _engine(case, hb)
+    for _ in range(2):  # the second call finds the ticket as the first left it
+        to_device(hb, db)
+        eng.fix_recovery(db)
+    case.oracle.fix_recovery(hb)
+    assert np.array_equal(field(db, "prim"), hb.prim)
+    assert np.array_equal(field(db, "flag"), hb.flag)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_cks_tables_or_not(precision):
+    """One mesh keeps its metric in tables, a pool forms it in the kernels."""
+    from pangu_b200.engine import Pool, Simulation
+    pin = problems.cks_atmosphere_input(n=20, nblock=10)
+    pin.set("b200", "precision", precision)
+    geo = problems.Geometry(prm.mesh_struct(pin))
+    prim = problems.cks_atmosphere(geo, prm.process_packages(pin))
+    sim = Simulation(pin)
+    sim.set_primitives(prim)
+    pool = Pool(pin, 9, 1)
+    job = pool.attach(pin, prim)
+    for _ in range(3):
+        sim.step()
+        pool.step(graph=False)
+    torch.cuda.synchronize()
+    assert np.array_equal(sim.primitives(), pool.primitives(job), equal_nan=True)
+    assert float(sim.dt) == float(pool.dt[job])
