@@ -2713,16 +2713,45 @@ __global__ void __launch_bounds__(kFixRecThreads) k_fixrec(Dims d, const int *co
 // its full transverse range, leaves every ghost cell equal to one interior
 // (or exchanged) cell, reached by applying each direction's rule in turn to
 // the index, with the reflections' sign flips composed. The kernel computes
-// that composition directly; its sources are never written by it.
+// that composition directly; its sources are never written by it. One thread per
+// ghost cell: the interior (three quarters of a 64^3 block) has none.
 // ---------------------------------------------------------------------------
+// Ghost cell t of a block: whole planes outside [ks, ke], then rows outside
+// [js, je], then the ends of the interior rows.
+__device__ __forceinline__ void ghost_cell(const Dims &d, long long t, int idx[3]) {
+  const int n1 = d.ie - d.is + 1, n2 = d.je - d.js + 1, n3 = d.ke - d.ks + 1;
+  const long long K = (long long)(d.N3 - n3) * d.N2 * d.N1, J = (long long)n3 * (d.N2 - n2) * d.N1;
+  long long r, i;
+  if (t < K) {
+    const int k = (int)div_fast(t, (long long)d.N2 * d.N1, r);
+    idx[2] = k < d.ks ? k : k + n3;
+    idx[1] = (int)div_fast(r, d.N1, i);
+    idx[0] = (int)i;
+  } else if (t < K + J) {
+    idx[2] = d.ks + (int)div_fast(t - K, (long long)(d.N2 - n2) * d.N1, r);
+    const int j = (int)div_fast(r, d.N1, i);
+    idx[1] = j < d.js ? j : j + n2;
+    idx[0] = (int)i;
+  } else {
+    idx[2] = d.ks + (int)div_fast(t - K - J, (long long)n2 * (d.N1 - n1), r);
+    idx[1] = d.js + (int)div_fast(r, d.N1 - n1, i);
+    idx[0] = (int)i < d.is ? (int)i : (int)i + n1;
+  }
+}
+inline __host__ __device__ long long ghost_cells(const Dims &d) {
+  return d.ncell - (long long)(d.ie - d.is + 1) * (d.je - d.js + 1) * (d.ke - d.ks + 1);
+}
+
 __global__ void __launch_bounds__(kThreads) k_bcs(Dims d, int enable_B, PT *P,
                                                   double *flag) {
   pdl_grid_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int bb, idx[3];
-  if (!box_index(t, d.NB, 0, d.N3 - 1, 0, d.N2 - 1, 0, d.N1 - 1, bb, idx[2], idx[1], idx[0]))
-    return;
-  const int b = slot_of(d, bb);
+  const long long per = ghost_cells(d);
+  if (t >= per * d.NB) return;
+  int idx[3];
+  long long g;
+  const int b = slot_of(d, (int)div_fast(t, per, g));
+  ghost_cell(d, g, idx);
   const signed char *bcf = d.bcf + 6 * b;  // -1 unless the face is a physical boundary
   const int st[3] = {d.is, d.js, d.ks}, en[3] = {d.ie, d.je, d.ke};
   int src[3] = {idx[0], idx[1], idx[2]};
@@ -2798,7 +2827,11 @@ __global__ void k_dt_init(int n, unsigned long long *mins) {
 }
 
 // One CTA row per mesh block (blockIdx.y); warp and CTA minima, then one
-// atomic per CTA and direction.
+// atomic per CTA and direction. Rounding is monotonic, so the smallest
+// cdx / speed of a thread's cells is the quotient of one of them: of the largest
+// speed, or, where a speed is negative, of the negative one nearest zero (whose
+// dt is the most negative). Speeds are compared by their bits (a NaN never
+// counts) and one division per direction follows.
 __device__ __forceinline__ void dt_reduce_cta(const Dims &d, double cfl, const double *alfven,
                                               unsigned long long *mins) {
   __shared__ unsigned long long red[3][kThreads / 32];
@@ -2810,18 +2843,43 @@ __device__ __forceinline__ void dt_reduce_cta(const Dims &d, double cfl, const d
   const double cdx[3] = {MUL(cfl, dx_of(d, b, 0)), MUL(cfl, dx_of(d, b, 1)),
                          MUL(cfl, dx_of(d, b, 2))};
   const int act[3] = {d.N1 > 1, d.N2 > 1, d.N3 > 1};
+  constexpr unsigned long long sign = 0x8000000000000000ull, inf = 0x7ff0000000000000ull;
+  // bits of the largest speed that is not negative, plus one (0: none), and of the
+  // negative speed nearest zero
+  unsigned long long pos[3] = {0, 0, 0}, neg[3] = {~0ull, ~0ull, ~0ull};
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < per;
        t += (long long)gridDim.x * blockDim.x) {
     int bz, k, j, i;
     box_index(t, 1, d.ks, d.ke, d.js, d.je, d.is, d.ie, bz, k, j, i);
+    const long long o = coff(d, k, j, i);
 #pragma unroll
     for (int dir = 0; dir < 3; ++dir) {
       if (!act[dir]) continue;
-      const double dt = cdx[dir] / a_alfven(d, alfven, b, dir)[coff(d, k, j, i)];
-      if (dt == dt) {
-        const unsigned long long key = dt_key(dt);
-        m[dir] = key < m[dir] ? key : m[dir];
+      const double speed = a_alfven(d, alfven, b, dir)[o];
+      if (!(cdx[dir] > 0.0)) {  // no order to rely on
+        const double dt = cdx[dir] / speed;
+        if (dt == dt) {
+          const unsigned long long key = dt_key(dt);
+          m[dir] = key < m[dir] ? key : m[dir];
+        }
+        continue;
       }
+      const unsigned long long v = (unsigned long long)__double_as_longlong(speed);
+      if ((v & ~sign) > inf) continue;  // NaN
+      if (v & sign)
+        neg[dir] = v < neg[dir] ? v : neg[dir];
+      else
+        pos[dir] = v + 1 > pos[dir] ? v + 1 : pos[dir];
+    }
+  }
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    if (!act[dir] || (pos[dir] == 0 && neg[dir] == ~0ull)) continue;
+    const unsigned long long v = neg[dir] != ~0ull ? neg[dir] : pos[dir] - 1;
+    const double dt = cdx[dir] / __longlong_as_double((long long)v);
+    if (dt == dt) {
+      const unsigned long long key = dt_key(dt);
+      m[dir] = key < m[dir] ? key : m[dir];
     }
   }
 #pragma unroll
@@ -3672,7 +3730,7 @@ int run_fix_recovery(pangu_engine *e, const pangu_pack *md, cudaStream_t s) {
 // Physical BCs of the blocks of d (all active blocks, or one job's).
 int run_bcs(pangu_engine *e, const Dims &d, bool any_bc, const pangu_pack *md, cudaStream_t s) {
   if (!any_bc || d.NB == 0) return PANGU_OK;
-  launch_pdl(k_bcs, dim3(grid_for((long long)d.NB * d.ncell)), dim3(kThreads), s, d, e->p.enable_B,
+  launch_pdl(k_bcs, dim3(grid_for(d.NB * ghost_cells(d))), dim3(kThreads), s, d, e->p.enable_B,
              prim_of(md), md->flag);
   ++e->launches;
   return check_launch();

@@ -139,3 +139,45 @@ def test_cks_tables_or_not(precision):
     torch.cuda.synchronize()
     assert np.array_equal(sim.primitives(), pool.primitives(job), equal_nan=True)
     assert float(sim.dt) == float(pool.dt[job])
+
+
+@pytest.mark.parametrize("cfl", [0.3, 0.0, -0.3])
+@pytest.mark.parametrize("kind", ["plain", "zeros", "negative", "nan", "inf"])
+def test_timestep_from_any_speeds(kind, cfl):
+    """The reference's minimum (timestep_estimation.cc:56-92) takes a negative dt and
+    skips a NaN."""
+    case = _case("ot", {("core", "cfl_number"): cfl}, n=40, nblock=20)
+    hb, _ = case.oracle_containers()
+    rng = np.random.default_rng(8)
+    a = rng.uniform(0.0, 2.0, hb.alfven.shape)
+    pick = rng.random(a.shape)
+    if kind == "zeros":
+        a[pick < 0.5], a[pick > 0.8] = 0.0, -0.0
+    elif kind == "negative":
+        a[pick < 0.3] *= -1.0
+    elif kind == "nan":
+        a[pick < 0.9] = np.nan
+    elif kind == "inf":
+        a[pick < 0.1] = np.inf
+    hb.alfven[...] = a
+    eng, db, _ = _engine(case, hb)
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    eng.estimate_dt(db, out)
+    geo = case.geo
+    big = np.finfo(np.float64).max
+    est = big
+    with np.errstate(all="ignore"):
+        for b in range(geo.nb):
+            inv = 0.0
+            for d in range(3):
+                m = np.float64(big)
+                if geo.act[d]:
+                    q = (cfl * geo.dx[d]) / hb.alfven[b, d][geo.interior()]
+                    q = q[~np.isnan(q)]
+                    m = np.float64(min(big, q.min())) if q.size else m
+                inv = np.float64(1.0) / m if d == 0 else inv + np.float64(1.0) / m
+            bdt = np.float64(1.0) / inv
+            est = bdt if bdt < est else est
+    # a minimum of zero may carry either sign, whose reciprocals differ
+    if not (np.isinf(est) or est == 0.0 or np.isnan(est)):
+        assert float(out) == float(est)
