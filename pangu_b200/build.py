@@ -26,8 +26,10 @@ INCLUDE = os.path.join(ROOT, "include")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "--fmad=false",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off", "-Xcompiler", "-O2",
-              # four threads per unit: 75 s instead of 4 min for engine.cu
-              "-split-compile=4", "-Xptxas", "-split-compile=4"]
+              # Four threads of ptxas per unit, whose code does not depend on them. (nvcc's
+              # own -split-compile gave one of two codes for the same engine.cu, kernels 8 %
+              # apart.)
+              "-Xptxas", "-split-compile=4"]
 
 
 # Translation units of the mixed-precision form: FMA contraction and the fast
