@@ -615,11 +615,14 @@ PGD double ppm4_face(double qm1, double q, double qp1, double qp2, bool &ok) {
   return b0 == b1 ? end : v;
 }
 // Upper-face value of a cell from its clamped face values; the lower-face
-// value is ppm4_side(q, up, lo). 2 x is exact, so q - 2 x is one rounding, and
-// the sign of |qc| - 2 |qd| rounded is the comparison's.
+// value is ppm4_side(q, up, lo). 2 x is exact, so q - 2 x is one rounding. The
+// comparison of the distances is ppm4's, which a NaN fails, so that a cell or face
+// values (ppm4_face_plain) that are not finite give ppm4's values too; a test of the
+// sign of |qc| - 2 |qd| does not. Staged x2 and x3 fluxes of a stage of the 3D torus:
+// 786 and 512 us, with the sign's test 796 and 519.
 PGD double ppm4_side(double q, double lo, double up) {
   const double qc = up - q, qd = lo - q;
-  const bool far = (int)xd::hi_bits(__fma_rn(-2.0, fabs(qd), fabs(qc))) >= 0;
+  const bool far = fabs(qc) >= 2.0 * fabs(qd);
   const double steep = far ? __fma_rn(-2.0, qd, q) : up;
   return (qc * qd) >= 0.0 ? q : steep;
 }

@@ -85,6 +85,50 @@ def test_fields_down_to_the_smallest_numbers(problem, kw, over):
         assert np.array_equal(field(do, f), getattr(ho, f), equal_nan=True), f
 
 
+SHAPES = ((1, 1, 128), (8, 2, 128), (1, 4, 128), (1, 0, 128), (1, 0, 256), (8, 8, 128))
+
+
+def _fluxes_of_every_shape(case, hb):
+    """(shape, field, result, oracle's result) of calculate_fluxes for each tile shape."""
+    eng, db, _ = _engine(case, hb)
+    case.oracle.calculate_fluxes(hb)
+    fields = ("flux1", "flux2", "alfven") + (("flux3",) if case.mesh.nx3 > 1 else ())
+    for m1, m, t in SHAPES:
+        eng.set_flux_config(x1_march=m1, x2_march=m, x2_threads=t, x3_march=m, x3_threads=t)
+        for f in fields:
+            getattr(db, f).zero_()
+        eng.calculate_fluxes(db)
+        for f in fields:
+            yield (m1, m, t), f, field(db, f), getattr(hb, f)
+
+
+def _some_not_finite(hb, seed):
+    """NaN anywhere; infinities, alone and in pairs of one sign along each direction, in
+    the scalars (where a component is structurally zero the oracle multiplies it out)."""
+    rng = np.random.default_rng(seed)
+    hb.prim[rng.random(hb.prim.shape) < 1e-3] = np.nan
+    for v in {0, 1, hb.prim.shape[1] - 2, hb.prim.shape[1] - 1} - {7}:
+        q = hb.prim[:, v]
+        for ax in (None, -1, -2, -3):
+            at = rng.random(q.shape) < 2e-3
+            q[at if ax is None else at | np.roll(at, 1, ax)] = rng.choice([np.inf, -np.inf])
+
+
+@pytest.mark.parametrize("problem,kw,over", [
+    ("torus", dict(nx1=58, nx2=24), {}),
+    ("torus", dict(nx1=26, nx2=16, nx3=8, bx=(26, 8, 8)), {}),
+    ("ot", dict(n=58), PPM4)])
+def test_ppm4_next_to_cells_that_are_not_finite(problem, kw, over):
+    """Every shape of the flux kernels limits a cell beside a NaN or an infinity as the
+    scalar limiter does, the staged tiles (march 8) among them."""
+    case = _case(problem, over, **kw)
+    hb, _ = case.oracle_containers()
+    _some_not_finite(hb, 9)
+    for shape, f, a, b in _fluxes_of_every_shape(case, hb):
+        assert np.isfinite(b).mean() > 0.3
+        assert np.array_equal(a, b, equal_nan=True), (shape, f)
+
+
 @pytest.mark.parametrize("model", sorted(abi.HEATING_MODEL))
 @pytest.mark.parametrize("suppress", [False, True])
 def test_heating_with_and_without_the_state(model, suppress):
