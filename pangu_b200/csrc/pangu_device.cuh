@@ -588,14 +588,15 @@ PGD bool state_speed(double gam, const double P[NPRIM], const Geo &g, const xd::
 // (qr_i) of the centre cell of a 3-point MC stencil.
 // The slope is minmod(a, b, c) with a = 2 (q - qm1), c = 2 (qp1 - q) and their
 // mean b. Where a and c have one sign so has b, and the smallest magnitude of
-// the three is the answer (0 when one of them is 0, so the signs' bits decide);
-// a NaN neighbour makes b, hence m, NaN and the slope 0.
+// the three is the answer (0 when one of them is 0, so the signs' bits decide).
+// A NaN among the values makes a or c NaN, and so does an infinite q beside an
+// equal infinity: the slope is 0, as the comparisons of the signs give it.
 PGD void mc(double qm1, double q, double qp1, double &ql_ip1, double &qr_i) {
   const double a = 2.0 * (q - qm1), b = 0.5 * (qp1 - qm1), c = 2.0 * (qp1 - q);
   double m = fabs(a) < fabs(c) ? a : c;
   m = fabs(m) <= fabs(b) ? m : b;
   const bool same = (int)(xd::hi_bits(a) ^ xd::hi_bits(c)) >= 0;
-  const double slope = same && m == m ? m : 0.0;
+  const double slope = same && a == a && c == c ? m : 0.0;
   ql_ip1 = q + 0.5 * slope;
   qr_i = q - 0.5 * slope;
 }

@@ -129,6 +129,18 @@ def test_ppm4_next_to_cells_that_are_not_finite(problem, kw, over):
         assert np.array_equal(a, b, equal_nan=True), (shape, f)
 
 
+@pytest.mark.parametrize("problem,kw,over", [
+    ("torus", dict(nx1=60, nx2=24, limiter="mc", riemann="hll"), {}),
+    ("ot", dict(n=60), {})])
+def test_mc_next_to_cells_that_are_not_finite(problem, kw, over):
+    case = _case(problem, over, **kw)
+    hb, _ = case.oracle_containers()
+    _some_not_finite(hb, 10)
+    for shape, f, a, b in _fluxes_of_every_shape(case, hb):
+        assert np.isfinite(b).mean() > 0.3
+        assert np.array_equal(a, b, equal_nan=True), (shape, f)
+
+
 @pytest.mark.parametrize("model", sorted(abi.HEATING_MODEL))
 @pytest.mark.parametrize("suppress", [False, True])
 def test_heating_with_and_without_the_state(model, suppress):
