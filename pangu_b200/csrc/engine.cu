@@ -113,7 +113,7 @@ int pangu_engine_destroy(pangu_engine *e) {
   cudaFree(e->d_fail_vals);
   cudaFree(e->d_dtmin);
   cudaFree(e->d_dt_ticket);
-  cudaFree(e->d_fix_ticket);
+  cudaFree(e->d_fix_sync);
   cudaFree(e->d_err);
   cudaFree(e->d_hsend);
   cudaFree(e->d_hrecv);
@@ -236,7 +236,7 @@ int pool_init(pangu_engine *e, int capacity, int max_jobs, bool one_mesh) {
   rc |= dalloc(&e->d_fail_vals, (size_t)e->fail_cap * d.NF);
   rc |= dalloc(&e->d_dtmin, 3 * (size_t)capacity);
   rc |= dalloc(&e->d_dt_ticket, 1);
-  rc |= dalloc(&e->d_fix_ticket, 1);
+  rc |= dalloc(&e->d_fix_sync, 3);
   rc |= dalloc(&e->d_err, 1);
   rc |= dalloc(&e->d_tmp_slots, capacity);
   rc |= dalloc(&e->d_genred, 3);
@@ -263,7 +263,7 @@ int pool_init(pangu_engine *e, int capacity, int max_jobs, bool one_mesh) {
   ok &= cudaMemset(e->d_slot_job, 0, (size_t)capacity * sizeof(int)) == cudaSuccess;
   ok &= cudaMemset(e->d_bcf, 0xff, 6 * (size_t)capacity) == cudaSuccess;  // -1: no BC
   ok &= cudaMemset(e->d_dt_ticket, 0, sizeof(unsigned int)) == cudaSuccess;
-  ok &= cudaMemset(e->d_fix_ticket, 0, sizeof(unsigned int)) == cudaSuccess;
+  ok &= cudaMemset(e->d_fix_sync, 0, 3 * sizeof(unsigned int)) == cudaSuccess;
   ok &= cudaMemset(e->d_err, 0, sizeof(int)) == cudaSuccess;
   k_dt_init<<<grid_for(3 * capacity), kThreads>>>(3 * capacity, e->d_dtmin);
   ok &= cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;

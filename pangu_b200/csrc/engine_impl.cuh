@@ -127,7 +127,7 @@ struct pangu_engine {
   int *d_err = nullptr;  // set by a kernel whose bounded wait gave up (0 otherwise)
   unsigned long long *d_dtmin = nullptr;  // [capacity][3]
   unsigned int *d_dt_ticket = nullptr;    // CTAs done in the current dt reduction
-  unsigned int *d_fix_ticket = nullptr;   // the same of the current FixRecovery
+  unsigned int *d_fix_sync = nullptr;     // [3]: the counters of k_fixrec
   long long launches = 0;  // kernels launched through this handle
   // Block sharding (one mesh over several GPUs): this engine holds the blocks
   // of `rank`; ghost cells whose source block is on another rank travel as

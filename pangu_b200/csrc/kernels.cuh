@@ -2644,67 +2644,131 @@ __global__ void __launch_bounds__(kThreads) k_fixrec_scan(Dims d, pangu_params p
   list[n] = fc;
 }
 
-// Both phases in one launch: every CTA computes the values of its cells from the
-// primitives and flags as they stand; the CTA that finishes last (a ticket taken
-// after a fence, no waiting) writes them all. Nothing fails in most stages, and a
-// launch that finds the list empty costs 3 us of a cycle's 70 to 300, so one
-// launch instead of two; the last CTA's 1024 threads write a thousand cells in
-// about 2 us.
+// Both phases in one launch: the CTAs compute the values from the primitives and
+// flags as they stand, and once all have (a counter raised after a fence) the values
+// are written. Nothing fails in most stages, and a launch that finds the list empty
+// costs 1.5 us of a cycle's 70 to 300, so one launch instead of two. A short list is
+// written by the CTA that finishes last; of a long one it hands out chunks, to itself
+// and to the CTAs that still wait for it. They wait for a bounded time and are not
+// needed: the last CTA writes whatever is left, so nothing depends on which CTAs run
+// together. A thread takes one component of a cell, or all of a list that fills the
+// GPU by its cells.
+// Bound by the latency of its scattered loads and stores. On lists of 1e3, 1e5 and 4e6
+// cells: 8 to 13, 24 to 30 and 357 us, against 8 to 15, 25 to 32 and 597 as two
+// launches and 14 to 38, 390 to 540 and 15500 with one CTA writing; nothing listed, 3.0
+// against 3.3 us for both stages of a cycle.
 constexpr int kFixRecThreads = 1024;
+constexpr int kFixRecAlone = 8;        // components a thread that the last CTA writes alone
+constexpr int kFixRecPolls = 1 << 14;  // of 64 ns and a load from L2 each
+
+// Components [v, v1) of list entry e: task t of n * parts.
+struct FixTask {
+  long long e;
+  int v, v1;
+  __device__ __forceinline__ FixTask(long long t, int n, int parts, int nf) {
+    v = (int)div_fast(t, n, e);
+    v1 = parts == 1 ? nf : v + 1;
+  }
+};
+
+__device__ __forceinline__ void fixrec_write(const Dims &d, long long t0, long long t1, int n,
+                                             int parts, const long long *list, const double *vals,
+                                             PT *P, double *flag, unsigned long long *cnt) {
+  for (long long t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+    FixTask q(t, n, parts, d.NF);
+    long long b, c;
+    split_cell(list[q.e], d.ncell, b, c);
+    if (q.v == 0) {
+      a_flag(d, flag, (int)b)[c] = 1;
+      count(cnt, job_of(d, (int)b), PANGU_CNT_FIXRECOVERY, true);
+    }
+    for (int v0 = q.v; v0 < q.v1; v0 += 5) {  // five loads before their stores
+      double w[5];
+#pragma unroll
+      for (int u = 0; u < 5; ++u)
+        if (v0 + u < q.v1)
+          w[u] = __ldcg(vals + (long long)(v0 + u) * n + q.e);  // other CTAs' stores: past L1
+#pragma unroll
+      for (int u = 0; u < 5; ++u) {
+        const int v = v0 + u;
+        if (v < q.v1) a_prim(d, P, (int)b, v)[c] = (v >= 2 && v < 5) ? PT(0) : (PT)w[u];
+      }
+    }
+  }
+}
+
+// sync: CTAs that have computed, chunks handed out, CTAs that have left; all 0
+// before and after.
 __global__ void __launch_bounds__(kFixRecThreads) k_fixrec(Dims d, const int *count_in,
                                                            const long long *list, PT *P,
                                                            double *flag, double *vals,
                                                            unsigned long long *cnt,
-                                                           unsigned int *ticket) {
+                                                           unsigned int *sync) {
   pdl_grid_wait();
   const int n = *count_in;
   if (n == 0) return;
-  const int off2 = d.js != d.je ? 1 : 0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long fc = list[t];
-    const long long b = fc / d.ncell;
-    const long long c = fc - b * d.ncell;
-    const long long sj = (long long)off2 * d.N1;
+  const long long sj = d.js != d.je ? d.N1 : 0;
+  const long long threads = (long long)gridDim.x * blockDim.x;
+  const int parts = n < threads ? d.NF : 1;
+  const long long tasks = (long long)n * parts;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tasks; t += threads) {
+    FixTask k(t, n, parts, d.NF);
+    long long b, c;
+    split_cell(list[k.e], d.ncell, b, c);
     const double *fb = a_flag(d, flag, (int)b) + c;
     auto fl = [&](long long o) { return (int)fb[o]; };
     const int pf1 = fl(sj - 1), pf2 = fl(sj), pf3 = fl(sj + 1), pf4 = fl(1);
     const int pf5 = fl(-sj + 1), pf6 = fl(-sj), pf7 = fl(-sj - 1), pf8 = fl(-1);
-    for (int v = 0; v < d.NF; ++v) {
+    const bool sides = pf2 && pf4 && pf6 && pf8, corners = pf1 && pf3 && pf5 && pf7;
+#pragma unroll 2
+    for (int v = k.v; v < k.v1; ++v) {
       const PT *q = a_prim(d, P, (int)b, v) + c;
       double val;
-      if (pf2 && pf4 && pf6 && pf8)
+      if (sides)
         val = 0.25 * (q[sj] + q[-sj] + q[-1] + q[1]);
-      else if (pf1 && pf3 && pf5 && pf7)
+      else if (corners)
         val = 0.25 * (q[sj + 1] + q[sj - 1] + q[-sj + 1] + q[-sj - 1]);
       else
         val = 0.125 * (q[sj - 1] + q[sj] + q[sj + 1] + q[1] + q[-sj + 1] + q[-sj] + q[-sj - 1] +
                        q[-1]);
-      vals[t * d.NF + v] = val;
+      vals[(long long)v * n + k.e] = val;
     }
   }
-  __shared__ bool last;
+  __shared__ unsigned before, chunk;
+  __shared__ bool ready;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) before = atomicAdd(&sync[0], 1u);
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    const long long fc = list[t];
-    const long long b = fc / d.ncell;
-    const long long c = fc - b * d.ncell;
-    double w[NPRIM];
-#pragma unroll
-    for (int v = 0; v < NPRIM; ++v)
-      if (v < d.NF) w[v] = __ldcg(vals + (long long)t * d.NF + v);  // other CTAs' stores: past L1
-#pragma unroll
-    for (int v = 0; v < NPRIM; ++v)
-      if (v < d.NF) a_prim(d, P, (int)b, v)[c] = (v >= 2 && v < 5) ? PT(0) : (PT)w[v];
-    a_flag(d, flag, (int)b)[c] = 1;
-    count(cnt, job_of(d, (int)b), PANGU_CNT_FIXRECOVERY, true);
+  const bool last = before == gridDim.x - 1;
+  if ((long long)n * d.NF <= kFixRecAlone * kFixRecThreads) {
+    if (!last) return;
+    __threadfence();
+    fixrec_write(d, 0, tasks, n, parts, list, vals, P, flag, cnt);
+    if (threadIdx.x == 0) sync[0] = 0u;
+    return;
   }
-  if (threadIdx.x == 0) *ticket = 0u;
+  if (threadIdx.x == 0) {
+    unsigned done = last ? gridDim.x : 0u;
+    for (int polls = 0; done < gridDim.x && polls < kFixRecPolls; ++polls) {
+      __nanosleep(64);
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(done) : "l"(sync) : "memory");
+    }
+    ready = done == gridDim.x;
+    __threadfence();
+  }
+  __syncthreads();
+  const int take = parts == 1 ? kFixRecThreads : 2 * kFixRecThreads;  // tasks of a chunk
+  while (ready) {
+    if (threadIdx.x == 0) chunk = atomicAdd(&sync[1], 1u);
+    __syncthreads();
+    const long long t0 = (long long)chunk * take;
+    __syncthreads();
+    if (t0 >= tasks) break;
+    fixrec_write(d, t0, min(t0 + take, tasks), n, parts, list, vals, P, flag, cnt);
+  }
+  if (threadIdx.x == 0 && atomicAdd(&sync[2], 1u) == gridDim.x - 1)
+    sync[0] = sync[1] = sync[2] = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -3689,8 +3753,8 @@ int run_fix_recovery(pangu_engine *e, const pangu_pack *md, bool listed, cudaStr
     k_fixrec_scan<<<grid_for(n), kThreads, 0, s>>>(d, e->p, md->flag, count, list);
     ++e->launches;
   }
-  launch_pdl(k_fixrec, dim3(64), dim3(kFixRecThreads), s, d, count, list, prim_of(md), md->flag,
-             e->d_fail_vals, e->d_cnt, e->d_fix_ticket);
+  launch_pdl(k_fixrec, dim3(device_sms()), dim3(kFixRecThreads), s, d, count, list, prim_of(md),
+             md->flag, e->d_fail_vals, e->d_cnt, e->d_fix_sync);
   ++e->launches;
   return check_launch();
 }

@@ -177,6 +177,49 @@ def test_fix_recovery_of_any_number_of_cells(share):
     assert np.array_equal(field(db, "flag"), hb.flag)
 
 
+def _repair(case, share, calls):
+    hb, _ = case.oracle_containers()
+    rng = np.random.default_rng(11)
+    hb.flag[...] = (rng.random(hb.flag.shape) >= share).astype(float)
+    eng, db, _ = _engine(case, hb)
+    for _ in range(calls):  # each finds the counters as the one before left them
+        to_device(hb, db)
+        eng.fix_recovery(db)
+    return hb, eng, db
+
+
+# 9 components a cell: 8192 tasks (910 cells) are the longest list that one CTA writes
+@pytest.mark.parametrize("n,share", [(96, 0.09), (96, 0.11), (96, 1.0), (512, 0.4), (512, 1.0)])
+def test_fix_recovery_of_short_and_long_lists(n, share):
+    case = _case("ot", {}, n=n)
+    hb, _, db = _repair(case, share, 3)
+    case.oracle.fix_recovery(hb)
+    assert np.array_equal(field(db, "prim"), hb.prim)
+    assert np.array_equal(field(db, "flag"), hb.flag)
+
+
+def test_fix_recovery_of_every_cell_is_spread_over_the_gpu():
+    """A list of 262,144 cells takes less time than two evaluations of the fluxes (it
+    moves a fifth of their bytes): one CTA that wrote it alone took ten."""
+    case = _case("ot", {}, n=512)
+    hb, eng, db = _repair(case, 1.0, 1)
+    one = torch.zeros_like(db.flag)
+
+    def clock(f):
+        best = np.inf
+        for _ in range(5):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            db.flag.copy_(one)
+            e[0].record()
+            f(db)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        return best
+
+    assert clock(eng.fix_recovery) < 2.0 * clock(eng.calculate_fluxes)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_cks_tables_or_not(precision):
     """One mesh keeps its metric in tables, a pool forms it in the kernels."""
