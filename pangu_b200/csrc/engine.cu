@@ -152,14 +152,14 @@ int validate_mesh(const pangu_params &p, const pangu_mesh &m) {
   return validate_shape(p, m);
 }
 
-// Allocates an empty pool of `capacity` block slots for up to `max_jobs`
-// jobs with the block shape of e->m.
 // Tables of the CKS metric for an engine of one mesh (a pool's capacity is not all
 // in use): 1.7 KB a cell, about twice the job's own arrays, against some 1,500
-// FP64 operations per metric evaluation, eight evaluations a cell and stage: 952
-// against 1403 us per cycle on 64^3 cells in blocks of 32^3 (geometric source 166
-// against 431). They are kept while they take at most an eighth of the memory that
-// is free; where they do not fit the kernels evaluate the metric, to the same bits.
+// FP64 operations per metric evaluation, eight evaluations a cell and stage: 872
+// against 1329 us per cycle on 64^3 cells in blocks of 32^3 (geometric source 126
+// against 429). They are kept while they take at most an eighth of the memory that
+// is free, since a program makes its containers, and other engines, after this one:
+// the job's arrays then find room several times over. Where the tables do not fit the
+// kernels form the metric (CKS_POINT), to the same bits.
 void cks_tables(pangu_engine *e) {
   const Dims &d = e->d;
   constexpr TabLayout T = tab_layout(CKS);
@@ -184,6 +184,8 @@ void cks_tables(pangu_engine *e) {
   }
 }
 
+// Allocates an empty pool of `capacity` block slots for up to `max_jobs`
+// jobs with the block shape of e->m.
 int pool_init(pangu_engine *e, int capacity, int max_jobs, bool one_mesh) {
   const pangu_params &p = e->p;
   pangu_mesh one = e->m;

@@ -184,7 +184,7 @@ __device__ __forceinline__ void gcov_at(const Dims &d, const pangu_params &p, in
     ks_code_gcov(map_pt(d, b, i, q1, j, q2), p.a, g);
   } else if (MT == BL) {
     bl_code_gcov(map_pt(d, b, i, q1, j, q2), p.a, g);
-  } else if (MT == CKS) {
+  } else if (is_cks(MT)) {
     cks_code_gcov(x[1], x[2], x[3], p.a, g);
   } else {
     minkowski_gcov(g);
@@ -207,7 +207,10 @@ __device__ __forceinline__ void gcov_at(const Dims &d, const pangu_params &p, in
 // The CKS metric depends on all three coordinates: its tables hold every entry of
 // every cell and face (gcov and the connection unsymmetric, as the dense
 // arithmetic leaves them) and exist where they fit (cks_tables in engine.cu);
-// otherwise the kernels form the metric at each point.
+// otherwise the kernels form the metric at each point, in instances of their own
+// (CKS_POINT): in one kernel with the loads, the metric formed by a call, a cycle of a
+// pool of 64^3 cells took 1586 us, against 1329 formed in place, and 961 against 872
+// with the tables.
 struct TabLayout {
   int nsym, ncon, nmet, nconn, ncen;
   int sym[4][4];      // slot of g_rc (r, c symmetric), -1 if structurally zero
@@ -347,25 +350,6 @@ __device__ __forceinline__ int analytic_geo(const Dims &d, const pangu_params &p
   return ok;
 }
 
-// analytic_geo of the CKS metric out of line, for engines without its tables.
-__device__ __noinline__ int cks_geo(double x, double y, double z, double a, Geo *o) {
-  Geo g;
-  cks_code_gcov(x, y, z, a, g.gcov);
-  const int ok = gj_invert(g.gcov, g.gcon);
-  g.gdet = determinant(g.gcov);
-  g.sg = sqrt(fabs(g.gdet));
-  g.alpha = 1.0 / sqrt(-g.gcon[0][0]);
-  *o = g;
-  return ok;
-}
-__device__ __forceinline__ int cks_geo_at(const pangu_params &p, double x, double y, double z,
-                                          Geo &g) {
-  Geo c;
-  const int ok = cks_geo(x, y, z, p.a, &c);
-  g = c;
-  return ok;
-}
-
 // ComputeMetricAtLocation (christoffel.h:53-62) at cell centre (b, k, j, i).
 // Returns 0 if the metric is singular.
 template <int MT>
@@ -375,11 +359,11 @@ __device__ __forceinline__ int cell_metric(const Dims &d, const pangu_params &p,
     constexpr TabLayout L = tab_layout(MT);
     return load_geo<MT>(d.ctab + tab_at(L.ncen, d.N2, d.N1, b, j, i), g);
   } else if (MT == CKS) {
-    if (d.ctab) {
-      constexpr TabLayout L = tab_layout(MT);
-      return load_geo<MT>(d.ctab + tab_at(L.ncen, d.N3 * d.N2, d.N1, b, k * d.N2 + j, i), g);
-    }
-    return cks_geo_at(p, xc(d, b, 0, i), xc(d, b, 1, j), xc(d, b, 2, k), g);
+    constexpr TabLayout L = tab_layout(MT);
+    return load_geo<MT>(d.ctab + tab_at(L.ncen, d.N3 * d.N2, d.N1, b, k * d.N2 + j, i), g);
+  } else if (MT == CKS_POINT) {
+    const double x[4] = {0.0, xc(d, b, 0, i), xc(d, b, 1, j), xc(d, b, 2, k)};
+    return analytic_geo<MT>(d, p, b, i, 0, j, 0, x, g);
   } else {
     minkowski_geo(g);
     return 1;
@@ -416,17 +400,17 @@ __device__ __forceinline__ int face_metric(const Dims &d, const pangu_params &p,
       return load_geo<MT>(d.f2tab + tab_at(L.nmet, d.N2 + 1, d.N1, b, j, i), g);
     return cell_metric<MT>(d, p, b, k, j, i, g);  // independent of x3
   } else if (MT == CKS) {
-    if (d.ctab) {
-      constexpr TabLayout L = tab_layout(MT);
-      const double *t =
-          dir == 1 ? d.f1tab + tab_at(L.nmet, d.N3 * d.N2, d.N1 + 1, b, k * d.N2 + j, i)
-          : dir == 2 ? d.f2tab + tab_at(L.nmet, d.N3 * (d.N2 + 1), d.N1, b, k * (d.N2 + 1) + j, i)
-                     : d.f3tab + tab_at(L.nmet, (d.N3 + 1) * d.N2, d.N1, b, k * d.N2 + j, i);
-      return load_geo<MT>(t, g);
-    }
-    return cks_geo_at(p, dir == 1 ? xf(d, b, 0, i) : xc(d, b, 0, i),
-                      dir == 2 ? xf(d, b, 1, j) : xc(d, b, 1, j),
-                      dir == 3 ? xf(d, b, 2, k) : xc(d, b, 2, k), g);
+    constexpr TabLayout L = tab_layout(MT);
+    const double *t =
+        dir == 1 ? d.f1tab + tab_at(L.nmet, d.N3 * d.N2, d.N1 + 1, b, k * d.N2 + j, i)
+        : dir == 2 ? d.f2tab + tab_at(L.nmet, d.N3 * (d.N2 + 1), d.N1, b, k * (d.N2 + 1) + j, i)
+                   : d.f3tab + tab_at(L.nmet, (d.N3 + 1) * d.N2, d.N1, b, k * d.N2 + j, i);
+    return load_geo<MT>(t, g);
+  } else if (MT == CKS_POINT) {
+    const double x[4] = {0.0, dir == 1 ? xf(d, b, 0, i) : xc(d, b, 0, i),
+                         dir == 2 ? xf(d, b, 1, j) : xc(d, b, 1, j),
+                         dir == 3 ? xf(d, b, 2, k) : xc(d, b, 2, k)};
+    return analytic_geo<MT>(d, p, b, i, 0, j, 0, x, g);
   } else {
     minkowski_geo(g);
     return 1;
@@ -545,7 +529,7 @@ __global__ void __launch_bounds__(kFixThreads, 6) k_fix_primitive(Dims d, pangu_
     r = T1[i];
     rho_floor = T1[8 * (d.N1 + 1) + i];
     eng_floor = T1[9 * (d.N1 + 1) + i];
-  } else if (MT == CKS) {
+  } else if (is_cks(MT)) {
     const double x = xc(d, b, 0, i), y = xc(d, b, 1, j), z = xc(d, b, 2, k);
     const double a2 = p.a * p.a;
     const double rad2 = x * x + y * y + z * z;
@@ -619,7 +603,7 @@ __global__ void __launch_bounds__(kFixThreads, 6) k_fix_primitive(Dims d, pangu_
     u3 = v3;
     ent = ef;
   }
-  if (MT == CKS && r < p.r_excise) {
+  if (is_cks(MT) && r < p.r_excise) {
     const double e_excise = p.pexcise / (gam - 1.0);
     pr = p.dexcise;
     pu = e_excise;
@@ -658,7 +642,7 @@ __global__ void __launch_bounds__(kFixThreads, 6) k_fix_primitive(Dims d, pangu_
     u2 *= f;
     u3 *= f;
   }
-  const bool excised = MT == CKS && r < p.r_excise;
+  const bool excised = is_cks(MT) && r < p.r_excise;
   const double rho_after = kmax(pr, small);
   const double e_excise = p.pexcise / (gam - 1.0);
   if (excised) {
@@ -1260,7 +1244,7 @@ constexpr int kFluxBlocks = 4;
 // and x3 1576 against 1758). Their arithmetic is spelled out, so the bound
 // changes no result.
 constexpr int flux_blocks(int mt, bool march) {
-  return !PGK_MIXED || mt == CKS ? kFluxBlocks : (march ? 5 : 7);
+  return !PGK_MIXED || is_cks(mt) ? kFluxBlocks : (march ? 5 : 7);
 }
 // FP64, curved metrics: one side's state in registers at a time
 // (face_flux_split; 47 against 49 us on the 2D torus, 2.41 against 2.52 ms on
@@ -2074,7 +2058,7 @@ __device__ __forceinline__ void metric_derivs(const Dims &d, const pangu_params 
 #pragma unroll
       for (int c = 0; c < 4; ++c) dg[a][r][c] = 0.0;
   double x[4] = {0.0, 0.0, 0.0, 0.0};
-  if (MT == CKS) {
+  if (is_cks(MT)) {
     x[1] = xc(d, b, 0, i);
     x[2] = xc(d, b, 1, j);
     x[3] = xc(d, b, 2, k);
@@ -2177,7 +2161,7 @@ __device__ __forceinline__ void source_cell(const Dims &d, const pangu_params &p
   double T[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) emt_from_state(p.adiabatic_index, pc, s, r, T[r]);
-  if (MT == MKS || MT == BL || (MT == CKS && d.ctab)) {
+  if (MT == MKS || MT == BL || MT == CKS) {
     // Christoffel symbols from the centre table; structural zeros skipped
     constexpr TabLayout L = tab_layout(MT);
     const double *cn =
@@ -2320,7 +2304,8 @@ __global__ void __launch_bounds__(kThreads) k_build_tables_cks(Dims d, pangu_par
                y = kind == 2 ? xf(d, b, 1, j) : xc(d, b, 1, j),
                z = kind == 3 ? xf(d, b, 2, k) : xc(d, b, 2, k);
   Geo g;
-  const int ok = cks_geo_at(p, x, y, z, g);
+  const double at[4] = {0.0, x, y, z};
+  const int ok = analytic_geo<CKS>(d, p, b, i, 0, j, 0, at, g);
   double *o = tab + tab_at(nc, R3 * R2, W, b, (int)kj, i);
 #pragma unroll
   for (int r = 0; r < 4; ++r)
@@ -2508,7 +2493,7 @@ __device__ __forceinline__ void recovery_cell(const Dims &d, const pangu_params 
   b = slot_of(d, b);
   const bool robuster = p.recovery == PANGU_RECOVERY_ROBUSTER;
   const long long fc = cidx(d, b, k, j, i);
-  if (MT == CKS) {
+  if (is_cks(MT)) {
     const double x = xc(d, b, 0, i), y = xc(d, b, 1, j), z = xc(d, b, 2, k);
     const double a2 = p.a * p.a;
     const double rad2 = x * x + y * y + z * z;
@@ -3240,12 +3225,20 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
   return launch_pdl_smem(kernel, grid, block, 0, s, args...);
 }
 
+// The metric that an engine's kernels are compiled for (DISPATCH_MT's first argument).
+inline int kernel_metric(const pangu_engine *e) {
+  static_assert(CKS_POINT != PANGU_METRIC_MKS && CKS_POINT != PANGU_METRIC_BL &&
+                CKS_POINT != PANGU_METRIC_CKS && CKS_POINT != PANGU_METRIC_MINKOWSKI);
+  return e->p.metric_type == PANGU_METRIC_CKS && !e->d_ctab ? CKS_POINT : e->p.metric_type;
+}
+
 #define DISPATCH_MT(mt, KERNEL, grid, stream, ...)                          \
   do {                                                                      \
     switch (mt) {                                                           \
       case PANGU_METRIC_MKS: launch_pdl(KERNEL<MKS>, dim3(grid), dim3(kThreads), stream, __VA_ARGS__); break; \
       case PANGU_METRIC_BL: launch_pdl(KERNEL<BL>, dim3(grid), dim3(kThreads), stream, __VA_ARGS__); break; \
       case PANGU_METRIC_CKS: launch_pdl(KERNEL<CKS>, dim3(grid), dim3(kThreads), stream, __VA_ARGS__); break; \
+      case CKS_POINT: launch_pdl(KERNEL<CKS_POINT>, dim3(grid), dim3(kThreads), stream, __VA_ARGS__); break; \
       default: launch_pdl(KERNEL<MINKOWSKI>, dim3(grid), dim3(kThreads), stream, __VA_ARGS__); break; \
     }                                                                       \
   } while (0)
@@ -3256,6 +3249,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
       case PANGU_METRIC_MKS: launch_pdl(KERNEL<MKS>, dim3(grid), dim3(threads), stream, __VA_ARGS__); break; \
       case PANGU_METRIC_BL: launch_pdl(KERNEL<BL>, dim3(grid), dim3(threads), stream, __VA_ARGS__); break; \
       case PANGU_METRIC_CKS: launch_pdl(KERNEL<CKS>, dim3(grid), dim3(threads), stream, __VA_ARGS__); break; \
+      case CKS_POINT: launch_pdl(KERNEL<CKS_POINT>, dim3(grid), dim3(threads), stream, __VA_ARGS__); break; \
       default: launch_pdl(KERNEL<MINKOWSKI>, dim3(grid), dim3(threads), stream, __VA_ARGS__); break; \
     }                                                                                        \
   } while (0)
@@ -3322,7 +3316,7 @@ int run_fix_primitive(pangu_engine *e, const pangu_pack *md, bool with_cons, cud
   const long long n = (long long)d.NB * d.ncell;
   // on the stage path (with_cons) the C2P retry and FixRecovery list counters
   // are zeroed here for Recovery
-  DISPATCH_MT_T(e->p.metric_type, k_fix_primitive, (unsigned)((n + kFixThreads - 1) / kFixThreads), kFixThreads,
+  DISPATCH_MT_T(kernel_metric(e), k_fix_primitive, (unsigned)((n + kFixThreads - 1) / kFixThreads), kFixThreads,
                 s, d, e->p, prim_of(md), e->d_cnt,
               md->cons, with_cons ? 1 : 0, PGK_MIXED ? 0 : 1,
               with_cons ? e->d_fail_count : nullptr, with_cons ? e->d_fix_count : nullptr);
@@ -3337,7 +3331,7 @@ int run_fix_primitive(pangu_engine *e, const pangu_pack *md, cudaStream_t s) {
 int run_calc_cons(pangu_engine *e, const Dims &d, const pangu_pack *md, bool with_b,
                   cudaStream_t s) {
   const long long n = box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie);
-  DISPATCH_MT(e->p.metric_type, k_calc_cons, grid_for(n), s, d, e->p, prim_of(md), md->cons,
+  DISPATCH_MT(kernel_metric(e), k_calc_cons, grid_for(n), s, d, e->p, prim_of(md), md->cons,
               with_b ? 1 : 0);
   ++e->launches;
   return check_launch();
@@ -3526,10 +3520,11 @@ void launch_flux_opt(const pangu_engine *e, const pangu_pack *md, int dir, int m
 
 int run_flux_dir(pangu_engine *e, const pangu_pack *md, int dir, int march, int threads,
                  cudaStream_t s) {
-  switch (e->p.metric_type) {
+  switch (kernel_metric(e)) {
     case PANGU_METRIC_MKS: launch_flux_opt<MKS>(e, md, dir, march, threads, s); break;
     case PANGU_METRIC_BL: launch_flux_opt<BL>(e, md, dir, march, threads, s); break;
     case PANGU_METRIC_CKS: launch_flux_opt<CKS>(e, md, dir, march, threads, s); break;
+    case CKS_POINT: launch_flux_opt<CKS_POINT>(e, md, dir, march, threads, s); break;
     default: launch_flux_opt<MINKOWSKI>(e, md, dir, march, threads, s); break;
   }
   e->launches += dir == 1 && x1_rest_lanes(e->d) ? 2 : 1;
@@ -3690,7 +3685,7 @@ int run_source(pangu_engine *e, const pangu_pack *md, double beta, const double 
   const Dims d = bind(e, md);
   if (e->p.metric_type == PANGU_METRIC_MINKOWSKI) return PANGU_OK;  // zero connection
   const long long n = box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie);
-  DISPATCH_MT(e->p.metric_type, k_source, grid_for(n), s, d, e->p, prim_of(md), md->cons, beta, dt);
+  DISPATCH_MT(kernel_metric(e), k_source, grid_for(n), s, d, e->p, prim_of(md), md->cons, beta, dt);
   ++e->launches;
   return check_launch();
 }
@@ -3706,7 +3701,7 @@ int run_recovery(pangu_engine *e, const pangu_pack *md, bool list_fix, cudaStrea
   if (e->p.recovery == PANGU_RECOVERY_CHAINER && (long long)grid <= 7LL * device_sms()) {
     // one wave: the chain in the same pass; the cells the whole chain fails
     // form FixRecovery's list (the stage path)
-    DISPATCH_MT_T(e->p.metric_type, k_recovery_chain, grid, kRecoveryThreads, s, d, e->p,
+    DISPATCH_MT_T(kernel_metric(e), k_recovery_chain, grid, kRecoveryThreads, s, d, e->p,
                   prim_of(md), md->cons, md->flag, e->d_cnt,
                   list_fix ? e->d_fix_count : nullptr, list_fix ? e->d_fix_list : nullptr);
     ++e->launches;
@@ -3714,12 +3709,12 @@ int run_recovery(pangu_engine *e, const pangu_pack *md, bool list_fix, cudaStrea
   }
   if (!list_fix && cudaMemsetAsync(e->d_fail_count, 0, sizeof(int), s) != cudaSuccess)
     return PANGU_ECUDA;
-  DISPATCH_MT_T(e->p.metric_type, k_recovery, grid, kRecoveryThreads, s, d, e->p, prim_of(md),
+  DISPATCH_MT_T(kernel_metric(e), k_recovery, grid, kRecoveryThreads, s, d, e->p, prim_of(md),
                 md->cons, md->flag, e->d_cnt, e->d_fail_count, e->d_fail_list);
   ++e->launches;
   if (e->p.recovery == PANGU_RECOVERY_CHAINER) {
     // one-warp CTAs: the few thousand retried cells spread over every SM
-    DISPATCH_MT_T(e->p.metric_type, k_recovery_retry, 8 * 148, 32, s, d, e->p, prim_of(md),
+    DISPATCH_MT_T(kernel_metric(e), k_recovery_retry, 8 * 148, 32, s, d, e->p, prim_of(md),
                   md->cons, md->flag, e->d_cnt, e->d_fail_count, e->d_fail_list,
                   list_fix ? e->d_fix_count : nullptr, list_fix ? e->d_fix_list : nullptr);
     ++e->launches;
@@ -3735,7 +3730,7 @@ int run_heating(pangu_engine *e, const pangu_pack *md, cudaStream_t s) {
   const Dims d = bind(e, md);
   if (!e->p.enable_heating) return PANGU_OK;
   const long long n = box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie);
-  DISPATCH_MT(e->p.metric_type, k_heating, grid_for(n), s, d, e->p, prim_of(md), md->cons);
+  DISPATCH_MT(kernel_metric(e), k_heating, grid_for(n), s, d, e->p, prim_of(md), md->cons);
   ++e->launches;
   return check_launch();
 }
@@ -3984,7 +3979,7 @@ int run_generate(pangu_engine *e, int job, const pangu_problem &pb, const pangu_
   const long long ne = (long long)d.NB * d.ncell;
   const long long ni = box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie);
   PT *P = prim_of(base);
-  DISPATCH_MT(p.metric_type, k_gen_cells, grid_for(ne), s, d, p, ga, P, e->d_genred);
+  DISPATCH_MT(kernel_metric(e), k_gen_cells, grid_for(ne), s, d, p, ga, P, e->d_genred);
   ++e->launches;
   if (torus) {
     k_gen_normalize<<<grid_for(ne), kThreads, 0, s>>>(d, P, e->d_genred);

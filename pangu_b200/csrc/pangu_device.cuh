@@ -27,7 +27,10 @@ namespace pgd {
 
 // variable_mnemonics.h:7-14
 enum { RHO, ENY, UX1, UX2, UX3, BX1, BX2, BX3, ENT, KEL, NPRIM };
-enum { MINKOWSKI = 0, BL = 1, CKS = 2, MKS = 3 };
+// CKS_POINT: the CKS metric in the kernels of an engine without its tables, which
+// form it at each point.
+enum { MINKOWSKI = 0, BL = 1, CKS = 2, MKS = 3, CKS_POINT = 4 };
+__host__ __device__ constexpr bool is_cks(int mt) { return mt == CKS || mt == CKS_POINT; }
 
 #define PGD __device__ __forceinline__
 

@@ -240,6 +240,30 @@ def test_cks_tables_or_not(precision):
     assert float(sim.dt) == float(pool.dt[job])
 
 
+def test_forming_the_cks_metric_in_a_pool_costs_little_more_than_its_tables():
+    """The fluxes of a pool, whose kernels form the metric, against those of a mesh that
+    keeps it in tables: 1.1 times as long. Formed by a call out of the kernel, 1.3."""
+    from pangu_b200.engine import Pool, Simulation
+    pin = problems.cks_atmosphere_input(n=64, nblock=32)
+    prim = problems.cks_atmosphere(problems.Geometry(prm.mesh_struct(pin)),
+                                   prm.process_packages(pin))
+    sim, pool = Simulation(pin), Pool(pin, 8, 1)
+    sim.set_primitives(prim)
+    pool.attach(pin, prim)
+    times = []
+    for x in (sim, pool):
+        best = np.inf
+        for _ in range(20):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            x.engine.calculate_fluxes(x.base)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        times.append(best)
+    assert times[1] < 1.2 * times[0]
+
+
 @pytest.mark.parametrize("cfl", [0.3, 0.0, -0.3])
 @pytest.mark.parametrize("kind", ["plain", "zeros", "negative", "nan", "inf"])
 def test_timestep_from_any_speeds(kind, cfl):
