@@ -1,7 +1,8 @@
 """The branch-free quotients of pangu_b200/csrc/exactdiv.h against `/`, compiled
-for the host (the same operations, with std::fma): random operands of the whole
-range, reciprocals from first approximations as poor as allowed, zero
-numerators, and quotients built to lie next to a rounding boundary."""
+for the host (the same operations, with std::fma; test_gpu_exactdiv.py has the
+device): random operands of the whole range, reciprocals from first approximations
+as poor as allowed, zero numerators, and quotients built to lie next to a rounding
+boundary."""
 import ctypes as C
 import os
 import subprocess
@@ -68,9 +69,9 @@ def test_random_operands(lib, ea, eb):
         assert ok.mean() > 0.999
 
 
-def test_quotients_next_to_a_rounding_boundary(lib):
-    """A 2^k - M B = K for small K: A / B is within |K| units of the midpoint M."""
-    rng = np.random.default_rng(2)
+def next_to_a_rounding_boundary(rng):
+    """Operands with A 2^k - M B = K for small K: A / B is within |K| units of the
+    midpoint M."""
     a, b = [], []
     for _ in range(20000):
         B = int(rng.integers(2 ** 52, 2 ** 53)) | 1
@@ -84,7 +85,13 @@ def test_quotients_next_to_a_rounding_boundary(lib):
                     a.append(float(A))
                     b.append(float(B))
     assert len(a) > 20000
-    assert _same(lib, np.array(a), np.array(b), rng).all()
+    return np.array(a), np.array(b)
+
+
+def test_quotients_next_to_a_rounding_boundary(lib):
+    rng = np.random.default_rng(2)
+    a, b = next_to_a_rounding_boundary(rng)
+    assert _same(lib, a, b, rng).all()
 
 
 def test_mantissas_of_ones_are_refused_or_right(lib):
