@@ -154,9 +154,9 @@ int validate_mesh(const pangu_params &p, const pangu_mesh &m) {
 
 // Tables of the CKS metric for an engine of one mesh (a pool's capacity is not all
 // in use): 1.7 KB a cell, about twice the job's own arrays, against some 1,500
-// FP64 operations per metric evaluation, eight evaluations a cell and stage: 872
-// against 1329 us per cycle on 64^3 cells in blocks of 32^3 (geometric source 126
-// against 429). They are kept while they take at most an eighth of the memory that
+// FP64 operations per metric evaluation, eight evaluations a cell and stage: 864
+// against 1295 us per cycle on 64^3 cells in blocks of 32^3 (geometric source 123
+// against 430). They are kept while they take at most an eighth of the memory that
 // is free, since a program makes its containers, and other engines, after this one:
 // the job's arrays then find room several times over. Where the tables do not fit the
 // kernels form the metric (CKS_POINT), to the same bits.

@@ -209,7 +209,7 @@ __device__ __forceinline__ void gcov_at(const Dims &d, const pangu_params &p, in
 // arithmetic leaves them) and exist where they fit (cks_tables in engine.cu);
 // otherwise the kernels form the metric at each point, in instances of their own
 // (CKS_POINT): in one kernel with the loads, the metric formed by a call, a cycle of a
-// pool of 64^3 cells took 1586 us, against 1329 formed in place, and 961 against 872
+// pool of 64^3 cells took 1586 us, against 1295 formed in place, and 961 against 864
 // with the tables.
 struct TabLayout {
   int nsym, ncon, nmet, nconn, ncen;
@@ -774,8 +774,8 @@ constexpr int kFluxHLL = 1, kFluxMC = 2;
 #define PGK_FLUX_MC(p) ((OPT & kFluxMC) != 0)
 #endif
 
-// The metric at a face. The FP64 kernels load it before they reconstruct, so
-// that its loads' latency passes meanwhile; the mixed form loads it in face_flux.
+// The metric at a face, which the FP64 kernels load once the face is reconstructed
+// (face_geo) and the mixed form in face_flux.
 struct FaceGeo {
 #if !PGK_MIXED
   Geo g;
@@ -1241,11 +1241,17 @@ constexpr int kFluxBlocks = 4;
 // The mixed form's tabulated-metric kernels need 72 registers with one face's
 // reconstruction in flight and 96 with a march; bounds that say so keep ptxas
 // from taking 80 and 108 (x1 947 against 1052 us per cycle on the 3D torus, x2
-// and x3 1576 against 1758). Their arithmetic is spelled out, so the bound
-// changes no result.
+// and x3 1576 against 1758). What cancels in a face, the states, speeds and flux
+// components, is spelled out (tfma and its like); the reconstruction and HLL's
+// denominator are plain operators, which the compiler may contract differently in
+// another kernel. The shapes and the packed last faces agree bit for bit as built
+// (tests/test_gpu_tiles.py, tests/test_gpu_branches.py).
 constexpr int flux_blocks(int mt, bool march) {
   return !PGK_MIXED || is_cks(mt) ? kFluxBlocks : (march ? 5 : 7);
 }
+// The staged x1 rows at 6 (80 registers, 86 without): 39 against 42 us per cycle on four
+// tori of uneven grids; at 7 they spill and are slower than without.
+constexpr int flux_tma_x1_blocks(int mt) { return !PGK_MIXED || is_cks(mt) ? kFluxBlocks : 6; }
 // FP64, curved metrics: one side's state in registers at a time
 // (face_flux_split; 47 against 49 us on the 2D torus, 2.41 against 2.52 ms on
 // the 3D one). Minkowski keeps both (its metric takes no registers).
@@ -1743,7 +1749,7 @@ inline size_t tma_x1_smem(int nf, bool split) {
 }
 
 template <int MT, int OPT>
-__global__ void __launch_bounds__(32 * kTmaRowsX1, kFluxBlocks)
+__global__ void __launch_bounds__(32 * kTmaRowsX1, flux_tma_x1_blocks(MT))
     k_flux_x1_tma(const __grid_constant__ CUtensorMap tm, Dims d, pangu_params p, int k0, int k1,
                   int j0, int j1, int i0, int i1, double *F, double *alfven, int *err) {
   extern __shared__ __align__(128) unsigned char dsm[];
@@ -2351,9 +2357,11 @@ __global__ void __launch_bounds__(kThreads) k_table_to_f32(Dims d, const double 
 // form computes the state and the heating in FT (FP32). Only the models that
 // read b^2 (and the suppression at high magnetisation) need the metric and the
 // state: the constant and the Sharma model skip both (187 to 104 us per stage on
-// the 3D torus, 10 to 7.4 on the 2D one).
+// the 3D torus, 10 to 7.4 on the 2D one). The mixed form fits 6 CTAs per SM (40
+// registers; 100 against 109 us per cycle on the 3D torus at 45).
+constexpr int heating_blocks(int mt) { return !PGK_MIXED || is_cks(mt) ? 4 : 6; }
 template <int MT>
-__global__ void __launch_bounds__(kThreads, 4) k_heating(Dims d, pangu_params p, PT *P,
+__global__ void __launch_bounds__(kThreads, heating_blocks(MT)) k_heating(Dims d, pangu_params p, PT *P,
                                                       const double *U) {
   pdl_grid_wait();
   int b, k, j, i;
@@ -2469,12 +2477,14 @@ __device__ __forceinline__ void c2p_write(const Dims &d, PT *P, int b, int k, in
 // cells. CHAIN = true: the failing lanes run Scheme1Dvsq and Scheme1D at
 // once (the retry pass's arithmetic, from the same inputs), and `list` (may
 // be null) receives the cells the whole chain fails, FixRecovery's list.
-// The chained form is used when the pass has at most 7 CTAs per SM: then the
-// few long chains overlap the rest of the wave instead of running as a
-// separate latency-bound launch (2D 512 x 256 torus at steady state: 0.387
-// against 0.403 ms per cycle), while on larger grids the registers the
-// chain adds (spills) cost more than the retry launch (3D torus 11.17
-// against 10.98 ms, 48-torus batch 7.15 against 7.05 ms).
+// The chained form is used when the pass has at most 7 CTAs per SM, one wave and a
+// little of a second: then the few long chains overlap the rest of the pass instead of
+// running as a separate latency-bound launch. Per cycle, chained against split, on the
+// 2D torus of 256 x 256 cells (3.5 CTAs per SM), 512 x 256 (6.9), 768 x 256 (10.4) and
+// 1024 x 256 (13.8): 253 / 258, 346 / 355, 478 / 480 and 545.6 / 545.3 us (untuned
+// shapes); mixed form 163 / 169, 218 / 231, 305 / 320 and 352 / 362. The gain
+// fades with the size (6 resident CTAs instead of 7); the line lies below where FP64 is
+// even.
 // Bound by the latency of the Newton steps' dependent FP64 operations. With the
 // steps' divisions branch-free (newton_2d_step), per cycle: 718 against 819 us on
 // the 3D torus (667 against 773 in the mixed form), the chained form 59.6 against
@@ -3699,8 +3709,8 @@ int run_recovery(pangu_engine *e, const pangu_pack *md, bool list_fix, cudaStrea
   const long long n = box_count(d.NB, d.ks, d.ke, d.js, d.je, d.is, d.ie);
   const unsigned grid = (unsigned)((n + kRecoveryThreads - 1) / kRecoveryThreads);
   if (e->p.recovery == PANGU_RECOVERY_CHAINER && (long long)grid <= 7LL * device_sms()) {
-    // one wave: the chain in the same pass; the cells the whole chain fails
-    // form FixRecovery's list (the stage path)
+    // the chain in the same pass (see k_recovery_chain); the cells the whole chain
+    // fails form FixRecovery's list (the stage path)
     DISPATCH_MT_T(kernel_metric(e), k_recovery_chain, grid, kRecoveryThreads, s, d, e->p,
                   prim_of(md), md->cons, md->flag, e->d_cnt,
                   list_fix ? e->d_fix_count : nullptr, list_fix ? e->d_fix_list : nullptr);

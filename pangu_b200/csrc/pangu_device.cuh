@@ -607,8 +607,9 @@ PGD void mc(double qm1, double q, double qp1, double &ql_ip1, double &qr_i) {
 // cells: the interpolant and its clamping between the adjacent cell values are
 // the same sums and comparisons seen from either cell. ppm4_face clears ok
 // where the stencil is not finite or the numerator too small for xd::div12; the
-// caller then uses ppm4 (or ppm4_face_plain) for that variable. Finite operands need no NaN rules, so the clamps are
-// plain compares and selects (a zero may keep the other sign).
+// caller then uses ppm4 (or ppm4_face_plain) for that variable. Finite operands need
+// no NaN rules, so the clamps are plain compares and selects. (Of two zeros of unlike
+// sign it takes one, as fmin and fmax may take either.)
 PGD double ppm4_face(double qm1, double q, double qp1, double qp2, bool &ok) {
   const double n = 7.0 * (q + qp1) - (qm1 + qp2);
   ok &= xd::in_range0(n);
@@ -727,6 +728,8 @@ PGD bool harm_utsq(const double prim[9], const Geo &g, double &utsq) {
 template <int MT>
 PGD void harm_velocity(const Harm &s, double Gamma, double W, double prim[9]) {
   constexpr Pattern PT = metric_pattern(MT);
+  // The sign of a zero quotient does not matter: the sums that make qt start from +0,
+  // so qt is never -0.
   const double fac = Gamma / (W + s.Bsq);
   const xd::Rcp iw = xd::rcp(W);
   double n[3], q[3];
